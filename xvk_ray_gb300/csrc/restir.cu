@@ -42,6 +42,12 @@ constexpr int kBlock = 128;   // raygen (one 16 x 8 tile per block)
 constexpr int kTraceBlock = XR_TRACE_BLOCK;   // persistent traversal kernels
 constexpr int kTraceBlockInst = XR_TRACE_BLOCK_INST;
 template <bool INST> constexpr int trace_block() { return INST ? kTraceBlockInst : kTraceBlock; }
+// The traversal's per-warp working sets: dynamic shared memory (above the 48 KB of static).
+template <bool INST> constexpr size_t trace_smem() { return (trace_block<INST>() / 32) * sizeof(TraceWarp<INST>); }
+template <bool INST> __device__ __forceinline__ TraceWarp<INST>& trace_warp() {
+    extern __shared__ float4 trace_smem_mem[];
+    return reinterpret_cast<TraceWarp<INST>*>(trace_smem_mem)[threadIdx.x >> 5];
+}
 constexpr int kShadeBlock = XR_SHADE_BLOCK;   // persistent shading kernel
 
 struct HitPayload {
@@ -613,7 +619,7 @@ __global__ void __launch_bounds__(trace_block<INST>(), 1) k_trace_paths(FrameArg
                                                         uint32_t* nonfinite, uint32_t pixel_is_record) {
     const uint32_t count = *(volatile const uint32_t*)count_ptr;
     trace_persistent<false, INST, BOUND>(
-        fa.sc, count, next,
+        trace_warp<INST>(), fa.sc, count, next,
         [&](uint32_t i) {
             float4 a = q0[i], b = q1[i];
             RayIn r;
@@ -1185,7 +1191,7 @@ template <bool INST>
 __global__ void __launch_bounds__(trace_block<INST>(), 1) k_trace_shadow(FrameArgs fa) {
     const uint32_t count = *(volatile const uint32_t*)&fa.counters[32];
     trace_persistent<true, INST>(
-        fa.sc, count, &fa.counters[kCntFetchShadow],
+        trace_warp<INST>(), fa.sc, count, &fa.counters[kCntFetchShadow],
         [&](uint32_t i) {
             const uint2 e = fa.shadow_q[i];
             const float4 g = fa.gb_pos_cur[e.x >> 5];
@@ -1215,7 +1221,7 @@ __global__ void __launch_bounds__(trace_block<INST>(), 1) k_trace_shadow(FrameAr
 __global__ void __launch_bounds__(kTraceBlock, 1) k_trace_nee(FrameArgs fa) {
     const uint32_t count = *(volatile const uint32_t*)&fa.counters[kCntCacheNee];
     trace_persistent<true>(
-        fa.sc, count < fa.cache_t_cap ? count : fa.cache_t_cap, &fa.counters[kCntFetchNee],
+        trace_warp<false>(), fa.sc, count < fa.cache_t_cap ? count : fa.cache_t_cap, &fa.counters[kCntFetchNee],
         [&](uint32_t i) {
             const float4 a = fa.cache_nee[(size_t)i * 3u], b = fa.cache_nee[(size_t)i * 3u + 1u];
             RayIn r;
@@ -1464,13 +1470,28 @@ uint32_t persistent_grid(int sm_count, bool compat) {
     return (uint32_t)(o * sm_count);
 }
 
+// Shared memory of the traversal kernels on the current device (once per context).
+cudaError_t configure_trace_kernels() {
+    const void* one[] = {(const void*)k_trace_paths<false, false>, (const void*)k_trace_paths<false, true>,
+                         (const void*)k_trace_shadow<false>, (const void*)k_trace_nee};
+    const void* two[] = {(const void*)k_trace_paths<true, false>, (const void*)k_trace_paths<true, true>,
+                         (const void*)k_trace_shadow<true>};
+    cudaError_t e = cudaSuccess;
+    for (const void* k : one)
+        if (!e) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trace_smem<false>());
+    for (const void* k : two)
+        if (!e) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trace_smem<true>());
+    return e;
+}
+
 uint32_t trace_grid(int sm_count, bool instances) {
     static int occ[2] = {0, 0};
     int& o = occ[instances ? 1 : 0];
     if (o == 0) {
         int v = 0;
-        if (instances) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_trace_paths<true, false>, kTraceBlockInst, 0);
-        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_trace_paths<false, false>, kTraceBlock, 0);
+        if (instances) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_trace_paths<true, false>, kTraceBlockInst,
+                                                                     trace_smem<true>());
+        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_trace_paths<false, false>, kTraceBlock, trace_smem<false>());
         o = v > 0 ? v : 4;
     }
     return (uint32_t)(o * sm_count);
@@ -1488,19 +1509,19 @@ void launch_initial(const FrameArgs& fa, uint32_t nb, cudaStream_t st, void (*af
         const uint32_t rec = (cache && b >= 2u) ? 1u : 0u;
         const bool bound = XR_CAMERA_BOUND_MARGIN > 0.0f && !fa.compat && b == 0u && fa.sc.n_nodes >= kCameraBoundMinNodes;
         if (fa.sc.n_inst && bound)
-            k_trace_paths<true, true><<<fa.grid_trace, kTraceBlockInst, 0, st>>>(a, a.q_in[0], a.q_in[1], fa.hits, fa.counters + b,
+            k_trace_paths<true, true><<<fa.grid_trace, kTraceBlockInst, trace_smem<true>(), st>>>(a, a.q_in[0], a.q_in[1], fa.hits, fa.counters + b,
                                                                     fa.counters + kCntFetchPath + b, fa.counters + kCntError,
                                                                     fa.counters + kCntNonFinite, rec);
         else if (fa.sc.n_inst)
-            k_trace_paths<true, false><<<fa.grid_trace, kTraceBlockInst, 0, st>>>(a, a.q_in[0], a.q_in[1], fa.hits, fa.counters + b,
+            k_trace_paths<true, false><<<fa.grid_trace, kTraceBlockInst, trace_smem<true>(), st>>>(a, a.q_in[0], a.q_in[1], fa.hits, fa.counters + b,
                                                                      fa.counters + kCntFetchPath + b, fa.counters + kCntError,
                                                                      fa.counters + kCntNonFinite, rec);
         else if (bound)
-            k_trace_paths<false, true><<<fa.grid_trace, kTraceBlock, 0, st>>>(a, a.q_in[0], a.q_in[1], fa.hits, fa.counters + b,
+            k_trace_paths<false, true><<<fa.grid_trace, kTraceBlock, trace_smem<false>(), st>>>(a, a.q_in[0], a.q_in[1], fa.hits, fa.counters + b,
                                                                      fa.counters + kCntFetchPath + b, fa.counters + kCntError,
                                                                      fa.counters + kCntNonFinite, rec);
         else
-            k_trace_paths<false, false><<<fa.grid_trace, kTraceBlock, 0, st>>>(a, a.q_in[0], a.q_in[1], fa.hits, fa.counters + b,
+            k_trace_paths<false, false><<<fa.grid_trace, kTraceBlock, trace_smem<false>(), st>>>(a, a.q_in[0], a.q_in[1], fa.hits, fa.counters + b,
                                                                       fa.counters + kCntFetchPath + b, fa.counters + kCntError,
                                                                       fa.counters + kCntNonFinite, rec);
         const bool nee = cache && b >= 1u && b + 1u < nb;
@@ -1508,7 +1529,7 @@ void launch_initial(const FrameArgs& fa, uint32_t nb, cudaStream_t st, void (*af
         if (fa.compat) k_shade<true><<<fa.grid_persistent, kShadeBlock, 0, st>>>(a, fa.ubo, b, nb);
         else k_shade<false><<<fa.grid_persistent, kShadeBlock, 0, st>>>(a, fa.ubo, b, nb);
         if (b == 1u && after_bounce1) after_bounce1(arg);   // bounce 1's records are complete
-        if (nee) k_trace_nee<<<fa.grid_trace, kTraceBlock, 0, st>>>(a);
+        if (nee) k_trace_nee<<<fa.grid_trace, kTraceBlock, trace_smem<false>(), st>>>(a);
     }
     if (nb < 2u && after_bounce1) after_bounce1(arg);
 }
@@ -1560,8 +1581,8 @@ void launch_spatial(const FrameArgs& fa, cudaStream_t st) {
     const uint32_t sblocks = (fa.N + sb - 1u) / sb;
     k_spatial_select<<<sblocks, sb, 0, st>>>(fa, fa.ubo);
     if (fa.visibility) {
-        if (fa.sc.n_inst) k_trace_shadow<true><<<fa.grid_trace, kTraceBlockInst, 0, st>>>(fa);
-        else k_trace_shadow<false><<<fa.grid_trace, kTraceBlock, 0, st>>>(fa);
+        if (fa.sc.n_inst) k_trace_shadow<true><<<fa.grid_trace, kTraceBlockInst, trace_smem<true>(), st>>>(fa);
+        else k_trace_shadow<false><<<fa.grid_trace, kTraceBlock, trace_smem<false>(), st>>>(fa);
     }
     k_spatial_resolve<<<sblocks, sb, 0, st>>>(fa, fa.ubo);
 }

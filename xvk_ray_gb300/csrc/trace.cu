@@ -18,8 +18,9 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace(DeviceScene sc, const flo
                                                        int32_t* __restrict__ prim, int32_t* __restrict__ inst,
                                                        float* __restrict__ t, float2* __restrict__ bary, uint32_t* fetch,
                                                        uint32_t* flags, unsigned long long* work) {
+    __shared__ TraceWarp<INST> warps[kTraceBlock / 32];
     trace_persistent<ANY, INST>(
-        sc, n, fetch,
+        warps[threadIdx.x >> 5], sc, n, fetch,
         [&](uint32_t i) {
             float4 a = rays[2 * i], b = rays[2 * i + 1];
             RayIn r;

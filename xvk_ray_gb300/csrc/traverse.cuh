@@ -45,45 +45,50 @@ __device__ __forceinline__ RayTri prep_ray(float3 o, float3 d) {
     return r;
 }
 
-// Returns true on a hit with tmin <= t <= tmax; writes t and (b1, b2).
-__device__ __forceinline__ bool hit_triangle(const RayTri& r, float3 v0, float3 v1, float3 v2, float tmin,
-                                             float tmax, float* t_out, float* b1, float* b2) {
-    float3 A = v0 - r.o, B = v1 - r.o, C = v2 - r.o;
-    float Akz = sel3(A, r.kz), Bkz = sel3(B, r.kz), Ckz = sel3(C, r.kz);
-    float Ax = sel3(A, r.kx) - r.Sx * Akz;
-    float Ay = sel3(A, r.ky) - r.Sy * Akz;
-    float Bx = sel3(B, r.kx) - r.Sx * Bkz;
-    float By = sel3(B, r.ky) - r.Sy * Bkz;
-    float Cx = sel3(C, r.kx) - r.Sx * Ckz;
-    float Cy = sel3(C, r.ky) - r.Sy * Ckz;
-    float U = Cx * By - Cy * Bx;
-    float V = Ax * Cy - Ay * Cx;
-    float W = Bx * Ay - By * Ax;
-    float Az = r.Sz * Akz, Bz = r.Sz * Bkz, Cz = r.Sz * Ckz;
-    if (U == 0.0f || V == 0.0f || W == 0.0f) {
-        double Ud = (double)Cx * (double)By - (double)Cy * (double)Bx;
-        double Vd = (double)Ax * (double)Cy - (double)Ay * (double)Cx;
-        double Wd = (double)Bx * (double)Ay - (double)By * (double)Ax;
-        if ((Ud < 0.0 || Vd < 0.0 || Wd < 0.0) && (Ud > 0.0 || Vd > 0.0 || Wd > 0.0)) return false;
-        double det = Ud + Vd + Wd;
+// The test of one triangle slot (12 floats: v0, primitive id, v1, -, v2, -) against a
+// ray given as {origin's components kx, ky, kz; tmin}, {Sx, Sy, Sz; kx | ky << 2 | kz << 4}:
+// the vertex components are loaded in the ray's order, so nothing is permuted after.
+// Returns true on a hit with tmin <= t <= tmax; writes t, (b1, b2) and the primitive.
+__device__ __forceinline__ bool hit_slot(float4 r0, float4 r1, const float* __restrict__ tri, float tmax, float* t_out,
+                                         float* b1, float* b2, int32_t* prim) {
+    const uint32_t k = __float_as_uint(r1.w);
+    const float *px = tri + (k & 3u), *py = tri + ((k >> 2) & 3u), *pz = tri + (k >> 4);
+    const float Akz = __ldg(pz) - r0.z, Bkz = __ldg(pz + 4) - r0.z, Ckz = __ldg(pz + 8) - r0.z;
+    const float Ax = (__ldg(px) - r0.x) - r1.x * Akz;
+    const float Ay = (__ldg(py) - r0.y) - r1.y * Akz;
+    const float Bx = (__ldg(px + 4) - r0.x) - r1.x * Bkz;
+    const float By = (__ldg(py + 4) - r0.y) - r1.y * Bkz;
+    const float Cx = (__ldg(px + 8) - r0.x) - r1.x * Ckz;
+    const float Cy = (__ldg(py + 8) - r0.y) - r1.y * Ckz;
+    const float U = Cx * By - Cy * Bx;
+    const float V = Ax * Cy - Ay * Cx;
+    const float W = Bx * Ay - By * Ax;
+    const float Az = r1.z * Akz, Bz = r1.z * Bkz, Cz = r1.z * Ckz;
+    float t;
+    if ((U == 0.0f) | (V == 0.0f) | (W == 0.0f)) {
+        const double Ud = (double)Cx * (double)By - (double)Cy * (double)Bx;
+        const double Vd = (double)Ax * (double)Cy - (double)Ay * (double)Cx;
+        const double Wd = (double)Bx * (double)Ay - (double)By * (double)Ax;
+        if (((Ud < 0.0) | (Vd < 0.0) | (Wd < 0.0)) & ((Ud > 0.0) | (Vd > 0.0) | (Wd > 0.0))) return false;
+        const double det = Ud + Vd + Wd;
         if (det == 0.0) return false;
-        double T = Ud * (double)Az + Vd * (double)Bz + Wd * (double)Cz;
-        float t = (float)(T / det);
-        if (!(t >= tmin && t <= tmax)) return false;
-        *t_out = t;
+        const double T = Ud * (double)Az + Vd * (double)Bz + Wd * (double)Cz;
+        t = (float)(T / det);
+        if (!((t >= r0.w) & (t <= tmax))) return false;
         *b1 = (float)(Vd / det);
         *b2 = (float)(Wd / det);
-        return true;
+    } else {
+        if (((U < 0.0f) | (V < 0.0f) | (W < 0.0f)) & ((U > 0.0f) | (V > 0.0f) | (W > 0.0f))) return false;
+        const float det = U + V + W;
+        if (det == 0.0f) return false;
+        const float T = U * Az + V * Bz + W * Cz;
+        t = T / det;
+        if (!((t >= r0.w) & (t <= tmax))) return false;
+        *b1 = V / det;
+        *b2 = W / det;
     }
-    if ((U < 0.0f || V < 0.0f || W < 0.0f) && (U > 0.0f || V > 0.0f || W > 0.0f)) return false;
-    float det = U + V + W;
-    if (det == 0.0f) return false;
-    float T = U * Az + V * Bz + W * Cz;
-    float t = T / det;
-    if (!(t >= tmin && t <= tmax)) return false;
     *t_out = t;
-    *b1 = V / det;
-    *b2 = W / det;
+    *prim = __float_as_int(__ldg(tri + 3));
     return true;
 }
 
@@ -109,11 +114,6 @@ __device__ __forceinline__ float3 xform_dir(float4 r0, float4 r1, float4 r2, flo
 __device__ __forceinline__ float3 xform_normal(float4 r0, float4 r1, float4 r2, float3 v) {
     return make_float3((r0.x * v.x + r1.x * v.y) + r2.x * v.z, (r0.y * v.x + r1.y * v.y) + r2.y * v.z,
                        (r0.z * v.x + r1.z * v.y) + r2.z * v.z);
-}
-
-__device__ __forceinline__ uint32_t byte_of(uint32_t w0, uint32_t w1, uint32_t i) {
-    uint32_t w = i < 4 ? w0 : w1;
-    return (w >> ((i & 3u) * 8u)) & 0xFFu;
 }
 
 }  // namespace xr

@@ -3,16 +3,19 @@
 // Software replacement of the hardware TraceRay (opaque triangles, no culling,
 // closest hit with ties to the lowest primitive id, or first hit for shadow
 // rays).  Each warp keeps 32 rays in flight; once at least refill_min lanes have
-// finished (or all have), the warp refills them from the ray queue with one
-// atomic (Aila and Laine, "Understanding the Efficiency of Ray Traversal on
-// GPUs", HPG 2009): the per-ray set-up (reciprocals, shear constants) then runs
-// for many lanes at once instead of one or two.  The loop follows Ylitie,
-// Karras and Laine, "Efficient Incoherent Ray Traversal on GPUs Through
+// finished (or all have), the warp stores their hits and refills them from the ray
+// queue with one atomic (Aila and Laine, "Understanding the Efficiency of Ray
+// Traversal on GPUs", HPG 2009): the per-ray set-up (reciprocals, shear constants)
+// then runs for many lanes at once instead of one or two.  The nodes are visited as
+// in Ylitie, Karras and Laine, "Efficient Incoherent Ray Traversal on GPUs Through
 // Compressed Wide BVHs" (HPG 2017): a lane holds one group of internal children
 // still to visit (base index, hit bits in near-to-far order, internal-child
-// mask) and one group of triangles; each iteration visits at most one node,
-// then tests triangles while enough lanes of the warp have some, and postpones
-// the rest onto the lane's stack otherwise.
+// mask) and each iteration visits at most one node.
+//
+// Triangle tests are decoupled from the lanes that find them: a lane appends the
+// triangles of a visited node to its warp's queue and goes on with its nodes; once a
+// warp's worth is queued (or too few lanes have nodes left to visit), every lane
+// takes one queued test, whichever lane's ray it belongs to.
 //
 // The triangle test and the box test are those of traverse.cuh (same arithmetic
 // as the CPU oracle); only the order of the work differs, which the closest-hit
@@ -22,16 +25,20 @@
 
 namespace xr {
 
-constexpr uint32_t kTriGroupBit = 0x80000000u;   // stack entry holds a triangle group
+constexpr uint32_t kTriGroupBit = 0x80000000u;   // stack entry holds a group of instances (two-level traversal)
 constexpr uint32_t kLevelBit = 0x40000000u;      // stack entry marks the return to the top-level BVH
-#ifndef XR_POSTPONE_BELOW
-#define XR_POSTPONE_BELOW 8
+#ifndef XR_TEST_BATCH
+#define XR_TEST_BATCH 32
 #endif
 #ifndef XR_REFILL_MIN
 #define XR_REFILL_MIN 8
 #endif
-constexpr int kPostponeBelow = XR_POSTPONE_BELOW;  // default: lanes; fewer testing triangles -> postpone
-constexpr int kRefillMin = XR_REFILL_MIN;          // default: idle lanes before a refill (swept 1..16: 1 is 9% slower)
+#ifndef XR_MIN_RUNNING
+#define XR_MIN_RUNNING 16
+#endif
+constexpr uint32_t kTestBatch = XR_TEST_BATCH;     // default: queued triangle tests that make a batch
+constexpr uint32_t kRefillMin = XR_REFILL_MIN;     // default: finished lanes before a refill
+constexpr uint32_t kMinRunning = XR_MIN_RUNNING;   // fewer lanes with nodes left: test what is queued
 constexpr float kMinDir = 1e-20f;                 // smallest direction component seen by the box test
 
 struct RayIn {
@@ -63,150 +70,307 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
     return r;
 }
 
-// LoadRay(i) -> RayIn; StoreHit(i, const HitRec&).  `next` is the fetch counter
-// (zeroed before the launch), `count` the number of rays, `err` the error word.
-// With `work` non-null (query kernels only) the node visits and triangle tests
-// are summed into work[0] and work[1]; with `nonfinite` non-null, the rays ended
-// early for a non-finite origin or direction are counted there.
+// Reciprocal within one ulp: enough for the box test, whose far planes are widened by
+// a relative 2e-6.
+__device__ __forceinline__ float rcp_box(float x) {
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Per-warp working set of the traversal in shared memory: the queue of triangle tests,
+// and per lane its ray as the triangle test wants it and the closest hit so far.
+constexpr uint32_t kTriQueue = 64;
+constexpr uint32_t kStackRing = 64;   // at most kStackSize groups are on a lane's stack
+template <bool INST>
+struct alignas(16) TraceWarp {
+    float4 ray0[32];             // the origin's components kx, ky, kz; tmin
+    float4 ray1[32];             // Sx, Sy, Sz; kx | ky << 2 | kz << 4
+    float2 bary[32];
+    uint32_t q_slot[kTriQueue];  // triangle slot of each queued test
+    float t[32];
+    int32_t prim[32];
+    uint8_t q_lane[kTriQueue];   // and the lane whose ray is tested
+    uint8_t winner[32];
+    int32_t inst[INST ? 32 : 4];
+};
+
+// LoadRay(i) -> RayIn; StoreHit(i, const HitRec&).  `sh` is the calling warp's working
+// set, `next` the fetch counter (zeroed before the launch), `count` the number of rays,
+// `err` the error word.  With `work` non-null (query kernels only) the node visits and
+// triangle tests are summed into work[0] and work[1]; with `nonfinite` non-null, the rays
+// ended early for a non-finite origin or direction are counted there.
 //
 // INST: two-level traversal of a scene with instances.  Rays start at the root of
-// the top-level BVH (sc.tlas_nodes), whose leaf slots are instances; "testing" one
+// the top-level BVH (sc.tlas_nodes), whose leaf slots are instances; entering one
 // saves the rest of the lane's top-level work on its stack under a level marker,
 // maps the ray into the instance's object space (origin and direction by its
 // world-to-object rows; t is unchanged) and continues at the root of its
-// bottom-level BVH in sc.nodes.  Popping the marker restores the world-space ray
-// (kept in the lane's registers or local memory since the ray's start).  Hits compare t, then instance, then primitive.
+// bottom-level BVH in sc.nodes.  Popping the marker, once no test of the lane is
+// queued any more, restores the world-space ray (kept in the lane's registers or
+// local memory since the ray's start).  Hits compare t, then instance, then primitive.
 //
 // RETRY (closest hit): a ray whose tmax is below retry_tmax treats its tmax
 // as a guess at where it hits.  Boxes beyond it are culled from the start; a ray that
 // ends without a hit inside it is traced again up to retry_tmax.  The result is the
 // same either way: when a hit lies within tmax, the closest hit (and every hit tied
 // with it) does too.
+//
+// Once the queue is empty, idle lanes help the warp's last rays (one-level traversal): a
+// lane with groups on its stack hands the bottom one, the largest part of what it has
+// left, to an idle lane with a copy of its ray.  Tests found by a helper go to the ray's
+// record, and a ray is finished when neither its lane nor a helper has anything left.
 template <bool ANY, bool INST = false, bool RETRY = false, typename LoadRay, typename StoreHit>
-__device__ __forceinline__ void trace_persistent(const DeviceScene& sc, uint32_t count, uint32_t* next,
-                                                 LoadRay load, StoreHit store, uint32_t* err,
+__device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const DeviceScene& sc, uint32_t count,
+                                                 uint32_t* next, LoadRay load, StoreHit store, uint32_t* err,
                                                  unsigned long long* work = nullptr, uint32_t* nonfinite = nullptr,
                                                  float retry_tmax = 0.0f) {
     static_assert(!RETRY || !ANY, "the retry is for closest-hit traversal");
-    const uint32_t FULL = 0xFFFFFFFFu;
-    uint32_t n_visits = 0, n_tests = 0, n_nonfinite = 0;
-    // queue tuning of the context (0: the defaults kRefillMin / kPostponeBelow)
-    const int refill_min = sc.refill_min ? (int)sc.refill_min : kRefillMin;
-    const int postpone_below = sc.postpone_below ? (int)sc.postpone_below : kPostponeBelow;
+    constexpr bool HELP = !INST;
+    constexpr uint32_t FULL = 0xFFFFFFFFu;
+    uint32_t n_visits = 0, n_tests = 0;
+    // queue tuning of the context (0: the defaults kRefillMin / kTestBatch)
+    const uint32_t refill_min = sc.refill_min ? sc.refill_min : kRefillMin;
+    const uint32_t batch = sc.postpone_below ? sc.postpone_below : kTestBatch;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt_mask = (1u << lane) - 1u;
-    bool active = false, drained = false;
-    bool retry = false;   // RETRY: the lane's ray is traced again up to retry_tmax on a miss
-    uint32_t ray_id = 0;
+    uint32_t q_head = 0, q_count = 0;   // the queue, a ring; these are the same in all lanes
+    uint32_t pending = 0;               // rays (their lanes) with a queued test
+    bool drained = false;
+    bool helping = false;                // lanes have been sent to help; the same in all lanes
+    uint32_t ray_id = kInvalid;          // the lane's ray (kInvalid: none)
+    uint32_t of = lane;                  // the lane whose ray it works on: its own, or the one it helps
+    bool retry = false;   // RETRY: it is traced again up to retry_tmax on a miss
     float3 o = f3(0, 0, 0);
-    float idx = 0, idy = 0, idz = 0, tmin = 0, tmin_box = 0;
-    RayTri rt;
+    float idx = 0, idy = 0, idz = 0, tmin_box = 0;
+    float h_t = 0;        // t of the closest hit so far (sh.t of this lane)
     uint32_t flip = 0;
-    HitRec h;
-    h.prim = -1; h.t = 0; h.b1 = 0; h.b2 = 0;
-    uint2 stack[kStackSize];
-    int sp = 0;
+    uint2 stack[kStackRing];
+    uint32_t sp = 0, sb = 0;             // a ring: the bottom moves up when a helper takes it
     uint32_t ng_base = 0, ng_bits = 0;   // bits 0..7 hits (near-to-far), 8..15 internal-child mask
     uint32_t tg_base = 0, tg_mask = 0;
-    uint32_t visits_left = 0;
-    bool bad = false;
     bool in_blas = !INST;    // INST: the lane's ray is in an instance's object space
     int32_t cur_inst = -1;   // that instance
-    h.inst = -1;
     // INST: the world-space ray and its box-test state, kept for instance entries
     // and for the return to the top level (no reload, no reciprocals recomputed)
     float3 wo = f3(0, 0, 0), wd = f3(0, 0, 0);
-    float widx = 0, widy = 0, widz = 0;
+    float w_tmin = 0, widx = 0, widy = 0, widz = 0;
     uint32_t wflip = 0;
-    // box-test reciprocals and sign bits of a direction (see the comment at the ray start)
+    // Box-test reciprocals of the direction with each component kept at least kMinDir in
+    // magnitude (sign kept): an exactly zero component would give an infinite reciprocal,
+    // and inf - inf in the per-node plane constants below is NaN, which drops that axis
+    // from every slab test and walks the whole tree.  The box test then follows a ray that
+    // departs from the true one by at most kMinDir * t, far inside the slack of the stored
+    // boxes, so no box holding a hit is culled; the triangle test uses the true direction.
+    // The sign bits select the near planes (so that -0 picks the same planes as its
+    // infinite reciprocal).
     auto set_dir = [&](float3 d) {
-        idx = 1.0f / copysignf(fmaxf(fabsf(d.x), kMinDir), d.x);
-        idy = 1.0f / copysignf(fmaxf(fabsf(d.y), kMinDir), d.y);
-        idz = 1.0f / copysignf(fmaxf(fabsf(d.z), kMinDir), d.z);
+        idx = rcp_box(copysignf(fmaxf(fabsf(d.x), kMinDir), d.x));
+        idy = rcp_box(copysignf(fmaxf(fabsf(d.y), kMinDir), d.y));
+        idz = rcp_box(copysignf(fmaxf(fabsf(d.z), kMinDir), d.z));
         flip = (__float_as_uint(d.x) >> 31) | ((__float_as_uint(d.y) >> 31) << 1) | ((__float_as_uint(d.z) >> 31) << 2);
+    };
+    // The lane's ray as every lane's triangle test reads it.
+    auto put_ray = [&](float3 ro, float3 rd, float rtmin) {
+        const RayTri r = prep_ray(ro, rd);
+        sh.ray0[lane] = make_float4(sel3(ro, r.kx), sel3(ro, r.ky), sel3(ro, r.kz), rtmin);
+        sh.ray1[lane] = make_float4(r.Sx, r.Sy, r.Sz, __uint_as_float((uint32_t)(r.kx | (r.ky << 2) | (r.kz << 4))));
+    };
+    // The virtual group whose only child is the first node to visit.
+    auto start_at = [&](uint32_t root, bool there) {
+        ng_base = root;
+        ng_bits = there ? (1u | ((1u << flip) << 8)) : 0u;
+    };
+    // The whole ray's start: at the top-level root, or at the root of its scene.
+    auto start_ray = [&](uint32_t root) {
+        if (INST) {
+            in_blas = false;
+            cur_inst = -1;
+            start_at(0u, sc.n_tlas_nodes != 0u);
+        } else {
+            start_at(root, root < sc.n_nodes);   // no root: a miss
+        }
+    };
+    // A bound was exceeded: the ray goes on without what lies beyond it, the call fails.
+    auto overflow = [&]() { atomicOr(err, (uint32_t)XR_DEVFLAG_STACK_OVERFLOW); };
+    // One queued test per lane, the oldest first (all lanes of the warp call this).
+    auto run_tests = [&]() {
+        __syncwarp();
+        const uint32_t k = min(q_count, 32u);
+        const uint32_t at = (q_head + lane) & (kTriQueue - 1u);
+        const bool on = lane < k;
+        const uint32_t owner = on ? sh.q_lane[at] : lane;
+        bool hit = false;
+        float tt = 0.0f, b1 = 0.0f, b2 = 0.0f;
+        int32_t prim = -1;
+        if (on) {
+            const uint32_t slot = sh.q_slot[at];
+            if (slot < sc.n_tri_slots) {
+                n_tests++;
+                hit = hit_slot(sh.ray0[owner], sh.ray1[owner], reinterpret_cast<const float*>(sc.tri + 3u * (size_t)slot),
+                               sh.t[owner], &tt, &b1, &b2, &prim);
+            } else {
+                overflow();
+            }
+        }
+        const int32_t r_inst = INST ? __shfl_sync(FULL, cur_inst, owner) : -1;
+        q_head = (q_head + k) & (kTriQueue - 1u);
+        q_count -= k;
+        // Merge: of the lanes whose hit beats a finder's record one writes it, until no
+        // lane's hit beats its record (several hits of one ray in one batch are rare).
+        // A record only ever improves, so the order of the tests does not matter; each
+        // round settles at least one lane, so at most 32 follow.
+        while (true) {
+            if (hit) {
+                const float ct = sh.t[owner];
+                const int32_t cp = sh.prim[owner];
+                bool tie_wins = prim < cp;
+                if (INST) {
+                    const int32_t ci = sh.inst[owner];
+                    tie_wins = r_inst < ci || (r_inst == ci && prim < cp);
+                }
+                hit = ANY ? cp < 0 : (cp < 0 ? tt <= ct : (tt < ct || (tt == ct && tie_wins)));
+            }
+            if (!__any_sync(FULL, hit)) break;
+            if (hit) sh.winner[owner] = (uint8_t)lane;
+            __syncwarp();
+            if (hit && sh.winner[owner] == lane) {
+                sh.t[owner] = tt;
+                sh.prim[owner] = prim;
+                sh.bary[owner] = make_float2(b1, b2);
+                if (INST) sh.inst[owner] = r_inst;
+                hit = false;
+            }
+            __syncwarp();
+        }
+        if (!ANY) h_t = sh.t[of];
+        else if (sh.prim[of] >= 0) { ng_bits = 0u; tg_mask = 0u; sp = sb = 0; }   // occluded: nothing left to visit
+        // rays that still have a test queued
+        const uint32_t left = lane < q_count ? 1u << sh.q_lane[(q_head + lane) & (kTriQueue - 1u)] : 0u;
+        pending = q_count ? __reduce_or_sync(FULL, left) : 0u;
     };
 
     while (true) {
-        // ---- refill idle lanes ----
-        const uint32_t idle = __ballot_sync(FULL, !active);
-        if (idle && !drained && (__popc(idle) >= refill_min || idle == FULL)) {
-            const uint32_t n_idle = __popc(idle);
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(next, n_idle);
-            base = __shfl_sync(FULL, base, 0);
-            if (base + n_idle >= count) drained = true;
-            if (!active) {
-                const uint32_t my = base + __popc(idle & lt_mask);
-                if (my < count) {
-                    RayIn r = load(my);
-                    ray_id = my;
-                    active = true;
-                    o = r.o;
-                    tmin = r.tmin;
-                    tmin_box = r.tmin * (1.0f - 1e-6f) - 1e-30f;
-                    // Box-test reciprocals of the direction with each component kept at
-                    // least kMinDir in magnitude (sign kept): an exactly zero component
-                    // would give an infinite reciprocal, and inf - inf in the per-node
-                    // plane constants below is NaN, which drops that axis from every slab
-                    // test and walks the whole tree.  The box test then follows a ray that
-                    // departs from the true one by at most kMinDir * t, far inside the
-                    // slack of the stored boxes, so no box holding a hit is culled;
-                    // the triangle test uses the true direction.
-                    // The sign bits select the near planes (so that -0 picks the same
-                    // planes as its infinite reciprocal).
-                    set_dir(r.d);
-                    rt = prep_ray(r.o, r.d);
-                    if (INST) { wo = r.o; wd = r.d; widx = idx; widy = idy; widz = idz; wflip = flip; }
-                    if constexpr (RETRY) retry = r.tmax < retry_tmax;
-                    h.prim = -1; h.t = r.tmax; h.b1 = 0.0f; h.b2 = 0.0f; h.inst = -1;
-                    sp = 0;
-                    tg_mask = 0;
-                    if (INST) {
-                        // every instance may be entered once: bound the visits accordingly
-                        const unsigned long long lim = ((unsigned long long)sc.n_nodes + sc.n_tlas_nodes) *
-                                                       (unsigned long long)max(sc.n_inst, 1u);
-                        visits_left = lim > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)lim;
-                        in_blas = false;
-                        cur_inst = -1;
-                        ng_base = 0u;   // the top-level root
-                        ng_bits = sc.n_tlas_nodes ? (1u | ((1u << flip) << 8)) : 0u;
+        const bool has_node = (ng_bits & 0xFFu) != 0u;
+        const uint32_t n_run = __popc(__ballot_sync(FULL, has_node || (INST && tg_mask)));
+        if (n_run + refill_min <= 32u) {
+            const bool empty = !(ng_bits & 0xFFu) && sp == sb && !(INST && tg_mask);
+            uint32_t busy = pending;   // rays with a queued test or a helper at work
+            if (HELP && helping) {
+                busy |= __reduce_or_sync(FULL, !empty && of != lane ? 1u << of : 0u);
+                if (empty) of = lane;
+            }
+            // finished rays are stored and idle lanes refilled, several at a time
+            const bool done = empty && !((busy >> lane) & 1u);
+            const uint32_t n_done = __popc(__ballot_sync(FULL, done));   // finished or idle
+            if (n_done == 32u || (n_done >= refill_min && (!drained || __any_sync(FULL, done && ray_id != kInvalid)))) {
+                if (done && ray_id != kInvalid) {
+                    if (RETRY && retry && sh.prim[lane] < 0) {
+                        // nothing within the first tmax: the same ray again from the root, up to
+                        // retry_tmax.  The lane holds the world-space ray here (an emptied stack
+                        // has popped every level marker), so its direction state is kept; the
+                        // triangle-test set-up of a one-level ray is kept too, and a two-level
+                        // ray sets it up again at each instance it enters.
+                        retry = false;
+                        h_t = retry_tmax;
+                        sh.t[lane] = retry_tmax;
+                        start_ray(INST ? 0u : load(ray_id).root);
                     } else {
-                        visits_left = sc.n_nodes;
-                        // a virtual group whose only child is the root (node 0)
-                        ng_base = r.root;
-                        ng_bits = (r.root < sc.n_nodes) ? (1u | ((1u << flip) << 8)) : 0u;   // no root: a miss
+                        HitRec h;
+                        h.prim = sh.prim[lane];
+                        h.t = sh.t[lane];
+                        const float2 b = sh.bary[lane];
+                        h.b1 = b.x; h.b2 = b.y;
+                        h.inst = INST ? sh.inst[lane] : -1;
+                        store(ray_id, h);
+                        ray_id = kInvalid;
                     }
-                    // A non-finite origin or direction (or a zero direction) can hit
-                    // nothing -- every triangle test fails -- but would make every box
-                    // test pass through NaN slabs and walk the whole tree: end it as a miss.
-                    const float chk = r.o.x + r.o.y + r.o.z + r.d.x + r.d.y + r.d.z;
-                    if (!isfinite(chk) || (r.d.x == 0.0f && r.d.y == 0.0f && r.d.z == 0.0f)) {
-                        ng_bits = 0u;
-                        n_nonfinite++;
-                        if constexpr (RETRY) retry = false;
+                }
+                const uint32_t idle = __ballot_sync(FULL, ray_id == kInvalid);
+                if (idle && !drained) {
+                    const uint32_t n_idle = __popc(idle);
+                    uint32_t base = 0;
+                    if (lane == 0) base = atomicAdd(next, n_idle);
+                    base = __shfl_sync(FULL, base, 0);
+                    if (base + n_idle >= count) drained = true;
+                    const uint32_t my = base + __popc(idle & lt_mask);
+                    if (ray_id == kInvalid && my < count) {
+                        const RayIn r = load(my);
+                        ray_id = my;
+                        o = r.o;
+                        tmin_box = r.tmin * (1.0f - 1e-6f) - 1e-30f;
+                        set_dir(r.d);
+                        if (INST) { wo = r.o; wd = r.d; w_tmin = r.tmin; widx = idx; widy = idy; widz = idz; wflip = flip; }
+                        else put_ray(r.o, r.d, r.tmin);
+                        if (RETRY) retry = r.tmax < retry_tmax;
+                        h_t = r.tmax;
+                        sh.t[lane] = r.tmax;
+                        sh.prim[lane] = -1;
+                        sh.bary[lane] = make_float2(0.0f, 0.0f);
+                        if (INST) sh.inst[lane] = -1;
+                        sp = sb = 0u;
+                        start_ray(r.root);
+                        // A non-finite origin or direction (or a zero direction) can hit
+                        // nothing -- every triangle test fails -- but would make every box
+                        // test pass through NaN slabs and walk the whole tree: end it as a miss.
+                        const float chk = r.o.x + r.o.y + r.o.z + r.d.x + r.d.y + r.d.z;
+                        if (!isfinite(chk) || (r.d.x == 0.0f && r.d.y == 0.0f && r.d.z == 0.0f)) {
+                            ng_bits = 0u;
+                            if (nonfinite) atomicAdd(nonfinite, 1u);
+                            if (RETRY) retry = false;
+                        }
                     }
+                }
+                if (!__any_sync(FULL, ray_id != kInvalid)) break;
+            }
+            if (HELP && drained) {
+                const bool idle = ray_id == kInvalid && of == lane;
+                const uint32_t m_idle = __ballot_sync(FULL, idle), m_give = __ballot_sync(FULL, sp != sb);
+                const uint32_t n = min(__popc(m_idle), __popc(m_give));
+                if (n) {   // the r-th idle lane takes from the r-th lane with a stack
+                    helping = true;
+                    const uint32_t r_give = __popc(m_give & lt_mask), r_take = __popc(m_idle & lt_mask);
+                    uint2 e = make_uint2(0u, 0u);
+                    if (sp != sb && r_give < n) {
+                        e = stack[sb++ & (kStackRing - 1u)];
+                        sh.winner[r_give] = (uint8_t)lane;
+                    }
+                    __syncwarp();
+                    const bool take = idle && r_take < n;
+                    const uint32_t from = take ? sh.winner[r_take] : lane;
+                    e.x = __shfl_sync(FULL, e.x, from);
+                    e.y = __shfl_sync(FULL, e.y, from);
+                    o.x = __shfl_sync(FULL, o.x, from);
+                    o.y = __shfl_sync(FULL, o.y, from);
+                    o.z = __shfl_sync(FULL, o.z, from);
+                    idx = __shfl_sync(FULL, idx, from);
+                    idy = __shfl_sync(FULL, idy, from);
+                    idz = __shfl_sync(FULL, idz, from);
+                    flip = __shfl_sync(FULL, flip, from);
+                    tmin_box = __shfl_sync(FULL, tmin_box, from);
+                    h_t = __shfl_sync(FULL, h_t, from);
+                    of = __shfl_sync(FULL, of, from);
+                    if (take) { ng_base = e.x; ng_bits = e.y; sp = sb = 0u; }
                 }
             }
         }
-        if (!__any_sync(FULL, active)) break;
 
-        // ---- node phase: visit the nearest remaining child of the current group ----
-        if (active && tg_mask == 0u && (ng_bits & 0xFFu)) {
+        // ---- visit the nearest remaining child of the current group ----
+        if (ng_bits & 0xFFu) {
             const uint32_t k = __ffs(ng_bits & 0xFFu) - 1u;
             ng_bits &= ~(1u << k);
             const uint32_t slot = k ^ flip;
             const uint32_t node = ng_base + __popc((ng_bits >> 8) & ((1u << slot) - 1u));
             if (ng_bits & 0xFFu) {
-                if (sp < kStackSize) stack[sp++] = make_uint2(ng_base, ng_bits);
-                else bad = true;
+                if (sp - sb < (uint32_t)kStackSize) stack[sp++ & (kStackRing - 1u)] = make_uint2(ng_base, ng_bits);
+                else overflow();
             }
             const WideNode* level_nodes = (INST && !in_blas) ? sc.tlas_nodes : sc.nodes;
             const uint32_t level_count = (INST && !in_blas) ? sc.n_tlas_nodes : sc.n_nodes;
-            if (node >= level_count || visits_left == 0u) {
-                bad = true;
+            if (node >= level_count) {
+                overflow();
                 ng_bits = 0;
             } else {
-                visits_left--;
                 n_visits++;
                 const uint4* np = reinterpret_cast<const uint4*>(level_nodes + node);
                 const uint4 w0 = __ldg(np + 0), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3),
@@ -218,7 +382,7 @@ __device__ __forceinline__ void trace_persistent(const DeviceScene& sc, uint32_t
                 const float ax = (__uint_as_float(w0.x) - o.x) * idx - sx;
                 const float ay = (__uint_as_float(w0.y) - o.y) * idy - sy;
                 const float az = (__uint_as_float(w0.z) - o.z) * idz - sz;
-                const float tlimit = h.t * (1.0f + 1e-6f) + 1e-30f;
+                const float tlimit = h_t * (1.0f + 1e-6f) + 1e-30f;
                 // near and far quantised planes per axis, chosen once per node from the
                 // sign bits of the direction (a negative axis enters through the high plane)
                 const bool nx = (flip & 1u) != 0u, ny = (flip & 2u) != 0u, nz = (flip & 4u) != 0u;
@@ -247,79 +411,79 @@ __device__ __forceinline__ void trace_persistent(const DeviceScene& sc, uint32_t
                 if (flip & 1u) ih = ((ih & 0x55u) << 1) | ((ih >> 1) & 0x55u);
                 if (flip & 2u) ih = ((ih & 0x33u) << 2) | ((ih >> 2) & 0x33u);
                 if (flip & 4u) ih = ((ih & 0x0Fu) << 4) | ((ih >> 4) & 0x0Fu);
+                // children come after their parent, so every descent ends
                 ng_base = w1.x;
                 ng_bits = ih | ((w0.w >> 24) << 8);
+                if (ih && w1.x <= node) { overflow(); ng_bits = 0u; }
                 tg_base = w1.y;
                 tg_mask = hm & 0x00FFFFFFu;
             }
         }
 
-        // ---- triangle phase: test while enough lanes have triangles ----
-        bool first = true;
-        while (true) {
-            const bool want = active && tg_mask != 0u;
-            const uint32_t m = __ballot_sync(FULL, want);
-            if (!m) break;
-            if (!first && (int)__popc(m) < postpone_below) {
-                if (want && sp < kStackSize) {
-                    stack[sp++] = make_uint2(tg_base, tg_mask | kTriGroupBit);
-                    tg_mask = 0u;
-                }
-                break;
-            }
-            first = false;
-            if (want && INST && !in_blas) {
-                // an instance: enter its bottom-level BVH in object space
-                const uint32_t bit = __ffs(tg_mask) - 1u;
-                tg_mask &= tg_mask - 1u;
-                if (tg_base + bit >= sc.n_inst_slots || sp + 3 > kStackSize) {
-                    bad = true;
-                    tg_mask = 0u;
-                    ng_bits = 0u;
-                } else {
-                    const float4* ip = sc.inst_slots + 4u * (tg_base + bit);
-                    const float4 m0 = __ldg(ip), m1 = __ldg(ip + 1), m2 = __ldg(ip + 2), m3 = __ldg(ip + 3);
-                    // the rest of the top-level work, then the level marker
-                    if (ng_bits & 0xFFu) stack[sp++] = make_uint2(ng_base, ng_bits);
-                    if (tg_mask) stack[sp++] = make_uint2(tg_base, tg_mask | kTriGroupBit);
-                    stack[sp++] = make_uint2(0u, kLevelBit);
-                    tg_mask = 0u;
-                    o = xform_point(m0, m1, m2, wo);
-                    const float3 od = xform_dir(m0, m1, m2, wd);
-                    set_dir(od);
-                    rt = prep_ray(o, od);
-                    cur_inst = (int32_t)__float_as_uint(m3.x);
-                    in_blas = true;
-                    ng_base = __float_as_uint(m3.y);
-                    const float chk = o.x + o.y + o.z + od.x + od.y + od.z;
-                    const bool ok = ng_base < sc.n_nodes && isfinite(chk) && !(od.x == 0.0f && od.y == 0.0f && od.z == 0.0f);
-                    ng_bits = ok ? (1u | ((1u << flip) << 8)) : 0u;
-                }
-            } else if (want) {
-                const uint32_t bit = __ffs(tg_mask) - 1u;
-                n_tests++;
-                tg_mask &= tg_mask - 1u;
-                if (tg_base + bit >= sc.n_tri_slots) {
-                    bad = true;
-                } else {
-                    const float4* tp = sc.tri + 3u * (tg_base + bit);
-                    const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
-                    const int32_t prim = (int32_t)__float_as_uint(a.w);
-                    float tt, b1, b2;
-                    const bool tie_wins = INST ? (cur_inst < h.inst || (cur_inst == h.inst && prim < h.prim))
-                                               : prim < h.prim;
-                    if (hit_triangle(rt, xyz(a), xyz(b), xyz(c), tmin, h.t, &tt, &b1, &b2) &&
-                        (h.prim < 0 || tt < h.t || (tt == h.t && tie_wins))) {
-                        h.prim = prim; h.t = tt; h.b1 = b1; h.b2 = b2; h.inst = cur_inst;
-                        if (ANY) { tg_mask = 0u; ng_bits = 0u; sp = 0; }
-                    }
-                }
+        // ---- instances found in a top-level node: enter one in object space ----
+        if (INST && !in_blas && tg_mask) {
+            const uint32_t bit = __ffs(tg_mask) - 1u;
+            tg_mask &= tg_mask - 1u;
+            if (tg_base + bit >= sc.n_inst_slots || sp + 3u > (uint32_t)kStackSize) {
+                overflow();
+                tg_mask = 0u;
+                ng_bits = 0u;
+            } else {
+                const float4* ip = sc.inst_slots + 4u * (tg_base + bit);
+                const float4 m0 = __ldg(ip), m1 = __ldg(ip + 1), m2 = __ldg(ip + 2), m3 = __ldg(ip + 3);
+                // the rest of the top-level work, then the level marker
+                if (ng_bits & 0xFFu) stack[sp++ & (kStackRing - 1u)] = make_uint2(ng_base, ng_bits);
+                if (tg_mask) stack[sp++ & (kStackRing - 1u)] = make_uint2(tg_base, tg_mask | kTriGroupBit);
+                stack[sp++ & (kStackRing - 1u)] = make_uint2(0u, kLevelBit);
+                tg_mask = 0u;
+                o = xform_point(m0, m1, m2, wo);
+                const float3 od = xform_dir(m0, m1, m2, wd);
+                set_dir(od);
+                put_ray(o, od, w_tmin);
+                cur_inst = (int32_t)__float_as_uint(m3.x);
+                in_blas = true;
+                const uint32_t root = __float_as_uint(m3.y);
+                const float chk = o.x + o.y + o.z + od.x + od.y + od.z;
+                start_at(root, root < sc.n_nodes && isfinite(chk) && !(od.x == 0.0f && od.y == 0.0f && od.z == 0.0f));
             }
         }
 
-        // ---- pop or finish ----
-        if (active && tg_mask == 0u && !(ng_bits & 0xFFu)) {
-            if (INST && sp > 0 && stack[sp - 1].y == kLevelBit) {
+        // ---- queue the triangles found ----
+        while (true) {
+            // up to three per lane where the ring has room (few nodes give a lane more), else one
+            const uint32_t n_tri = (!INST || in_blas) ? __popc(tg_mask) : 0u;
+            const uint32_t three = n_tri < 3u ? n_tri : 3u;
+            const uint32_t p0 = __ballot_sync(FULL, three & 1u), p1 = __ballot_sync(FULL, three & 2u);
+            uint32_t total = __popc(p0) + 2u * __popc(p1);
+            bool more = false;
+            if (total) {
+                uint32_t at = q_head + q_count + __popc(p0 & lt_mask) + 2u * __popc(p1 & lt_mask), n = three;
+                if (q_count + total > kTriQueue) {
+                    total = __popc(p0 | p1);
+                    at = q_head + q_count + __popc((p0 | p1) & lt_mask);
+                    n = three ? 1u : 0u;
+                }
+    #pragma unroll
+                for (uint32_t i = 0; i < 3; i++) {
+                    if (i < n) {
+                        sh.q_slot[(at + i) & (kTriQueue - 1u)] = tg_base + (__ffs(tg_mask) - 1u);
+                        sh.q_lane[(at + i) & (kTriQueue - 1u)] = (uint8_t)of;
+                        tg_mask &= tg_mask - 1u;
+                    }
+                }
+                q_count += total;
+                pending |= HELP && helping ? __reduce_or_sync(FULL, n ? 1u << of : 0u) : p0 | p1;
+                more = __any_sync(FULL, tg_mask != 0u && (!INST || in_blas));
+            }
+            // a whole batch, or what there is when too few lanes have nodes to visit
+            while (q_count >= batch || (!more && q_count && n_run < kMinRunning)) run_tests();
+            if (!more) break;
+        }
+
+        // ---- next group of nodes from the stack ----
+        if (!(ng_bits & 0xFFu) && sp != sb) {
+            uint2 e = stack[(sp - 1u) & (kStackRing - 1u)];
+            if (INST && e.y == kLevelBit && !((pending >> lane) & 1u)) {
                 // back to the top level: the world-space ray, then (same step) the
                 // top-level work saved under the marker -- markers are never adjacent
                 --sp;
@@ -328,43 +492,15 @@ __device__ __forceinline__ void trace_persistent(const DeviceScene& sc, uint32_t
                 flip = wflip;
                 in_blas = false;
                 cur_inst = -1;
+                e = sp ? stack[(sp - 1u) & (kStackRing - 1u)] : make_uint2(0u, 0u);
             }
-            bool again = false;
-            if constexpr (RETRY) again = sp == 0 && retry && h.prim < 0;
-            if (again) {
-                // nothing within the first tmax: the same ray again from the root, up to
-                // retry_tmax.  The lane holds the world-space ray here (an emptied stack
-                // has popped every level marker), so its direction state is kept; the
-                // triangle-test set-up of a one-level ray is kept too, and a two-level
-                // ray sets it up again at each instance it enters.
-                retry = false;
-                h.t = retry_tmax;
-                if (INST) {
-                    const unsigned long long lim = ((unsigned long long)sc.n_nodes + sc.n_tlas_nodes) *
-                                                   (unsigned long long)max(sc.n_inst, 1u);
-                    visits_left = lim > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)lim;
-                    in_blas = false;
-                    cur_inst = -1;
-                    ng_base = 0u;   // the top-level root
-                    ng_bits = sc.n_tlas_nodes ? (1u | ((1u << flip) << 8)) : 0u;
-                } else {
-                    visits_left = sc.n_nodes;
-                    const uint32_t root = load(ray_id).root;
-                    ng_base = root;
-                    ng_bits = (root < sc.n_nodes) ? (1u | ((1u << flip) << 8)) : 0u;
-                }
-            } else if (sp == 0) {
-                store(ray_id, h);
-                active = false;
-            } else {
-                const uint2 e = stack[--sp];
-                if (e.y & kTriGroupBit) { tg_base = e.x; tg_mask = e.y & 0x00FFFFFFu; ng_bits = 0u; }
+            if (sp != sb && !(INST && e.y == kLevelBit)) {
+                --sp;
+                if (INST && (e.y & kTriGroupBit)) { tg_base = e.x; tg_mask = e.y & 0x00FFFFFFu; }
                 else { ng_base = e.x; ng_bits = e.y; }
             }
         }
     }
-    if (__any_sync(FULL, bad) && bad) atomicOr(err, (uint32_t)XR_DEVFLAG_STACK_OVERFLOW);
-    if (n_nonfinite && nonfinite) atomicAdd(nonfinite, n_nonfinite);
     if (work) {
         atomicAdd(&work[0], (unsigned long long)n_visits);
         atomicAdd(&work[1], (unsigned long long)n_tests);

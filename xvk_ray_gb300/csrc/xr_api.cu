@@ -334,6 +334,7 @@ xr_status xr_create(const XrDeviceDesc* desc, XrContext** out) {
     if ((s = cuda_check(c, cudaGetDeviceProperties(&prop, c->device), "device properties"))) goto bad;
     if (prop.major < 10) { s = fail(c, XR_ERR_UNSUPPORTED, "create: this library is built for sm_103a (GB300)"); goto bad; }
     c->sm_count = prop.multiProcessorCount;
+    if ((s = cuda_check(c, configure_trace_kernels(), "traversal kernels"))) goto bad;
     if ((s = cuda_check(c, cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking), "stream"))) goto bad;
     if ((s = cuda_check(c, cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking), "copy stream"))) goto bad;
     if ((s = cuda_check(c, cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking), "side stream"))) goto bad;
@@ -840,7 +841,7 @@ xr_status xr_autotune(XrContext* c, const XrUniformBufferObject* ubos, uint32_t 
         {&c->tune_trace_ctas, fractions(occ_t)},                       // persistent traversal CTAs per SM
         {&c->tune_shade_ctas, fractions(occ_s)},                       // persistent shading CTAs per SM
         {&c->tune_refill, {0u, 4u, 6u, 12u, 16u}},                     // ray-queue refill: idle lanes per fetch
-        {&c->tune_postpone, {0u, 4u, 12u, 16u}},                       // triangle tests postponed below this many lanes
+        {&c->tune_postpone, {0u, 8u, 16u, 24u}},                       // queued triangle tests that make a batch
         {&c->tune_bundle, {0u, 1u, 2u}},                               // camera-ray bundle: 8x4, 16x2, 4x8 pixels
         {&c->tune_temporal_block, {0u, 32u, 128u, 256u}},              // temporal pass block (default 64)
         {&c->tune_spatial_block, {0u, 64u, 256u}},                     // spatial passes' block (default 128)

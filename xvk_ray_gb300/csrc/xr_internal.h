@@ -113,7 +113,7 @@ struct DeviceScene {
     const float4* inst_xform;        // 6 float4 per instance: object-to-world rows, world-to-object rows
     uint32_t n_inst;                 // 0: no instances
     // traversal queue tuning (xr_set_tuning / xr_autotune): idle lanes before a warp refills
-    // from the ray queue, and lanes with triangles below which a warp postpones its tests
+    // from the ray queue, and queued triangle tests that make a batch
     uint32_t refill_min, postpone_below;
 };
 
@@ -423,6 +423,7 @@ void launch_trace(const DeviceScene& sc, const float* rays, uint32_t n, int any_
                   cudaStream_t st);
 
 // ---- launch wrappers (restir.cu) ----
+cudaError_t configure_trace_kernels();   // per device, before the first frame
 // after_bounce1(arg), when given, is called once bounce 1's shading is enqueued (or after the
 // loop for a single bounce): the enqueue point of work that needs only bounce 1's records.
 void launch_initial(const FrameArgs& fa, uint32_t number_of_bounces, cudaStream_t st,
