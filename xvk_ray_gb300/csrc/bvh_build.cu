@@ -4,18 +4,21 @@
 // reference (ApplicationRT.cpp:186-258, XVKBLGeometry.cpp:8-38,
 // XVKAccelerationStructure.cpp:15-96: one opaque BLAS per model, identity
 // instances).  Steps, all on the context stream:
-//   1. per-triangle bounds, scene centroid bounds (warp reductions + atomics)
+//   1. per-triangle bounds, scene centroid bounds (block reductions + atomics)
 //   2. 63-bit Morton codes of the box centres (21 bits per axis)
-//   3. stable LSD radix sort of (code, primitive) pairs, 8 passes of 8 bits
-//   4. Karras, "Maximizing Parallelism in the Construction of BVHs, Octrees and
-//      k-d Trees" (HPG 2012) binary radix tree; equal codes split by index
-//   5. bottom-up bounds, second arrival at a node computes its box
-//   6. top-down collapse, one level per launch: each wide node takes up to 8
-//      children by repeatedly opening the child of largest surface area
-//      (subtrees of more than 3 triangles first), children of <= 3 triangles
-//      become leaves, slots are assigned by octant of the child centre so that a
-//      ray visits near children first, boxes are quantised to 8 bits (rounded
-//      outwards, plus the slack of kBoxSlackCells).
+//   3. stable LSD radix sort of (code, primitive) pairs, 8 passes of 8 bits (up to 2048
+//      pairs: one block)
+//   4. the binary tree: PLOC clustering (below), or with XR_BVH_BUILDER=lbvh and for
+//      instances Karras, "Maximizing Parallelism in the Construction of BVHs, Octrees and
+//      k-d Trees" (HPG 2012), whose radix tree splits equal codes by index and gets its
+//      bounds bottom-up, the second arrival at a node computing its box
+//   5. the SAH decisions of the collapse, bottom-up
+//   6. top-down collapse, one level per launch, eight lanes per wide node: the children the
+//      decisions give, children of <= 3 triangles become leaves, slots are assigned by
+//      octant of the child centre so that a ray visits near children first, boxes are
+//      quantised to 8 bits (rounded outwards, plus the slack of kBoxSlackCells).
+// The kernels hand their counts on through device words (BuildWords); the host waits once
+// per batch of clustering rounds and once per batch of levels.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -53,14 +56,40 @@ __host__ __device__ __forceinline__ float o2f(uint32_t u) {
 #endif
 }
 
-// bounds[0..2] centroid min, [3..5] centroid max, [6] largest |coordinate|
-// Primitive boxes: triangles from their vertices, or given boxes (box_lo non-null).
-__global__ void k_tri_prep(const uint4* __restrict__ tri_idx, const float4* __restrict__ vpos, uint32_t ntri,
-                           const float4* __restrict__ box_lo, const float4* __restrict__ box_hi,
-                           float4* __restrict__ tri_lo, float4* __restrict__ tri_hi, uint32_t* __restrict__ bounds) {
-    uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    float cmin[3] = {INFINITY, INFINITY, INFINITY}, cmax[3] = {-INFINITY, -INFINITY, -INFINITY}, amax = 0.0f;
-    if (t < ntri) {
+// Words of one build on the device: what the kernels share and the host reads back once.
+constexpr uint32_t kBuildLevels = 208;
+struct BuildWords {
+    uint32_t bounds[8];        // [0..2] centroid min, [3..5] centroid max (ordered), [6] largest |coordinate|
+    uint32_t counters[4];      // [0] wide nodes, [1] triangle slots, [3] inconsistencies found
+    uint32_t clusters[2];      // clusters left, by parity of the clustering round
+    uint32_t made;             // binary nodes made by the clustering
+    uint32_t root;             // root of the binary tree
+    uint32_t level_count[kBuildLevels];   // wide nodes of each level
+};
+
+__global__ void k_build_init(BuildWords* w, uint32_t n, uint32_t root) {
+    for (uint32_t i = threadIdx.x; i < sizeof(BuildWords) / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(w)[i] = 0u;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < 3; k++) w->bounds[k] = 0xFFFFFFFFu;
+        w->counters[0] = 1u;
+        w->clusters[0] = n;
+        w->root = root;
+        w->level_count[0] = 1u;
+    }
+}
+
+// Primitive boxes: triangles from their vertices, or given boxes (box_lo non-null).  The
+// bounds are reduced per block before the atomics: one set per warp serialised on seven
+// addresses (1M triangles: 144 us; 152 x 4 blocks: 13 us).
+constexpr int kPrepBlock = 256;
+__global__ void __launch_bounds__(kPrepBlock) k_tri_prep(const uint4* __restrict__ tri_idx, const float4* __restrict__ vpos,
+                                                         uint32_t ntri, const float4* __restrict__ box_lo,
+                                                         const float4* __restrict__ box_hi, float4* __restrict__ tri_lo,
+                                                         float4* __restrict__ tri_hi, uint32_t* __restrict__ bounds) {
+    __shared__ float part[kPrepBlock / 32][7];
+    float v[7] = {INFINITY, INFINITY, INFINITY, INFINITY, INFINITY, INFINITY, 0.0f};   // min, -max, -(-amax)
+    for (uint32_t t = blockIdx.x * kPrepBlock + threadIdx.x; t < ntri; t += gridDim.x * kPrepBlock) {
         float3 lo, hi;
         if (box_lo) {
             lo = xyz(box_lo[t]);
@@ -73,25 +102,30 @@ __global__ void k_tri_prep(const uint4* __restrict__ tri_idx, const float4* __re
         }
         tri_lo[t] = make_float4(lo.x, lo.y, lo.z, 0.0f);
         tri_hi[t] = make_float4(hi.x, hi.y, hi.z, 0.0f);
-        float cx = (lo.x + hi.x) * 0.5f, cy = (lo.y + hi.y) * 0.5f, cz = (lo.z + hi.z) * 0.5f;
-        cmin[0] = cmax[0] = cx; cmin[1] = cmax[1] = cy; cmin[2] = cmax[2] = cz;
-        amax = fmaxf(fmaxf(fmaxf(fabsf(lo.x), fabsf(lo.y)), fmaxf(fabsf(lo.z), fabsf(hi.x))),
-                     fmaxf(fabsf(hi.y), fabsf(hi.z)));
+        const float c[3] = {(lo.x + hi.x) * 0.5f, (lo.y + hi.y) * 0.5f, (lo.z + hi.z) * 0.5f};
+        for (int k = 0; k < 3; k++) {
+            v[k] = fminf(v[k], c[k]);
+            v[3 + k] = fminf(v[3 + k], -c[k]);
+        }
+        const float amax = fmaxf(fmaxf(fmaxf(fabsf(lo.x), fabsf(lo.y)), fmaxf(fabsf(lo.z), fabsf(hi.x))),
+                                 fmaxf(fabsf(hi.y), fabsf(hi.z)));
+        v[6] = fminf(v[6], -amax);
     }
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        for (int k = 0; k < 3; k++) {
-            cmin[k] = fminf(cmin[k], __shfl_xor_sync(0xFFFFFFFFu, cmin[k], off));
-            cmax[k] = fmaxf(cmax[k], __shfl_xor_sync(0xFFFFFFFFu, cmax[k], off));
+    for (int k = 0; k < 7; k++)
+        for (int off = 16; off > 0; off >>= 1) v[k] = fminf(v[k], __shfl_xor_sync(0xFFFFFFFFu, v[k], off));
+    if ((threadIdx.x & 31) == 0)
+        for (int k = 0; k < 7; k++) part[threadIdx.x >> 5][k] = v[k];
+    __syncthreads();
+    if (threadIdx.x < 7) {
+        const int k = threadIdx.x;
+        float m = part[0][k];
+        for (int w = 1; w < kPrepBlock / 32; w++) m = fminf(m, part[w][k]);
+        if (k == 6) atomicMax(&bounds[6], __float_as_uint(-m));
+        else if (m < INFINITY) {
+            if (k < 3) atomicMin(&bounds[k], f2o(m));
+            else atomicMax(&bounds[k], f2o(-m));
         }
-        amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, off));
-    }
-    if ((threadIdx.x & 31) == 0 && cmin[0] <= cmax[0]) {
-        for (int k = 0; k < 3; k++) {
-            atomicMin(&bounds[k], f2o(cmin[k]));
-            atomicMax(&bounds[3 + k], f2o(cmax[k]));
-        }
-        atomicMax(&bounds[6], __float_as_uint(amax));
     }
 }
 
@@ -138,32 +172,61 @@ __global__ void k_sort_hist(const uint64_t* __restrict__ keys, uint32_t n, uint3
     for (int i = threadIdx.x; i < 256; i += blockDim.x) hist[i * nblocks + b] = h[i];
 }
 
-// exclusive scan of hist[256 * nblocks] in one block
-__global__ void k_sort_scan(uint32_t* __restrict__ hist, uint32_t total) {
-    __shared__ uint32_t part[1024];
-    uint32_t per = (total + blockDim.x - 1) / blockDim.x;
-    uint32_t beg = threadIdx.x * per, end = min(total, beg + per);
-    uint32_t s = 0;
-    for (uint32_t i = beg; i < end; i++) s += hist[i];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t acc = 0;
-        for (uint32_t i = 0; i < blockDim.x; i++) { uint32_t v = part[i]; part[i] = acc; acc += v; }
+// Exclusive scan of each digit's row of block counts (one block per digit); the row's
+// total goes to tot[digit], whose scan is left to the scatter (one block scanning all rows
+// took 54 us a pass at 1M keys, this 5).
+__global__ void __launch_bounds__(kSortThreads) k_sort_rows(uint32_t* __restrict__ hist, uint32_t* __restrict__ tot,
+                                                            uint32_t nblocks) {
+    __shared__ uint32_t wsum[kSortThreads / 32];
+    uint32_t* row = hist + (size_t)blockIdx.x * nblocks;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t run = 0;
+    for (uint32_t base = 0; base < nblocks; base += kSortThreads) {
+        const uint32_t i = base + threadIdx.x;
+        const uint32_t v = i < nblocks ? row[i] : 0u;
+        uint32_t x = v;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, d);
+            if ((int)lane >= d) x += y;
+        }
+        if (lane == 31u) wsum[warp] = x;
+        __syncthreads();
+        uint32_t before = run, all = 0;
+        for (uint32_t w = 0; w < kSortThreads / 32; w++) {
+            if (w < warp) before += wsum[w];
+            all += wsum[w];
+        }
+        if (i < nblocks) row[i] = before + x - v;
+        run += all;
+        __syncthreads();
     }
-    __syncthreads();
-    uint32_t acc = part[threadIdx.x];
-    for (uint32_t i = beg; i < end; i++) { uint32_t v = hist[i]; hist[i] = acc; acc += v; }
+    if (threadIdx.x == 0) tot[blockIdx.x] = run;
 }
 
 __global__ void __launch_bounds__(kSortThreads) k_sort_scatter(const uint64_t* __restrict__ kin,
                                                                const uint32_t* __restrict__ vin, uint64_t* __restrict__ kout,
                                                                uint32_t* __restrict__ vout, uint32_t n, uint32_t chunk, int shift,
-                                                               const uint32_t* __restrict__ hist, uint32_t nblocks) {
+                                                               const uint32_t* __restrict__ hist,
+                                                               const uint32_t* __restrict__ tot, uint32_t nblocks) {
     __shared__ uint32_t base[256];
     __shared__ uint32_t wcnt[kSortThreads / 32][256];
+    __shared__ uint32_t wsum[kSortThreads / 32];
     const uint32_t b = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) base[i] = hist[i * nblocks + b];
+    {   // thread d: where digit d starts, and in it this block's share
+        const uint32_t v = tot[threadIdx.x];
+        uint32_t x = v;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, d);
+            if ((int)lane >= d) x += y;
+        }
+        if (lane == 31u) wsum[warp] = x;
+        __syncthreads();
+        uint32_t before = 0;
+        for (uint32_t w = 0; w < warp; w++) before += wsum[w];
+        base[threadIdx.x] = before + x - v + hist[threadIdx.x * nblocks + b];
+    }
     const uint32_t beg = b * chunk, end = min(n, beg + chunk);
     for (uint32_t tile = beg; tile < end; tile += kSortThreads) {
         for (int i = threadIdx.x; i < (kSortThreads / 32) * 256; i += blockDim.x) (&wcnt[0][0])[i] = 0;
@@ -191,6 +254,36 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_scatter(const uint64_t* _
             base[d] += tot;
         }
         __syncthreads();
+    }
+}
+
+// Up to kSmallSort keys in one block (bitonic, ties by index like the stable radix sort):
+// the top-level tree of a few hundred instances would otherwise spend 24 launches on it.
+constexpr uint32_t kSmallSort = 2048;
+__global__ void __launch_bounds__(1024) k_sort_small(uint64_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t n) {
+    __shared__ uint64_t k[kSmallSort];
+    __shared__ uint32_t v[kSmallSort];
+    uint32_t size = 2;
+    while (size < n) size <<= 1;
+    for (uint32_t i = threadIdx.x; i < size; i += blockDim.x) {
+        k[i] = i < n ? keys[i] : ~0ull;      // Morton codes have 63 bits
+        v[i] = i;
+    }
+    __syncthreads();
+    for (uint32_t span = 2; span <= size; span <<= 1)
+        for (uint32_t step = span >> 1; step; step >>= 1) {
+            for (uint32_t t = threadIdx.x; t < size / 2; t += blockDim.x) {
+                const uint32_t a = 2u * t - (t & (step - 1u)), b = a + step;
+                const uint64_t ka = k[a], kb = k[b];
+                const uint32_t va = v[a], vb = v[b];
+                const bool up = (a & span) == 0u, more = ka > kb || (ka == kb && va > vb);
+                if (more == up) { k[a] = kb; k[b] = ka; v[a] = vb; v[b] = va; }
+            }
+            __syncthreads();
+        }
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+        keys[i] = k[i];
+        vals[i] = v[i];
     }
 }
 
@@ -272,11 +365,11 @@ struct CollapseArgs {
     const float4* records;            // non-null: leaves copy 4 float4 per primitive from here (instances)
     const uint8_t* dec;               // non-null: wide nodes follow the SAH decisions of k_sah_dp
     const uint32_t* ref_prim;         // non-null: primitives are triangle pieces; the triangle of each
-    const uint32_t* task_in; const uint32_t* task_wide_in; uint32_t n_tasks;
+    const uint32_t* task_in; const uint32_t* task_wide_in;
     uint32_t* task_out; uint32_t* task_wide_out;
-    uint32_t* counters;               // [0] wide nodes, [1] tri slots, [2] next task count
+    BuildWords* words;
     WideNode* nodes; float4* tris;
-    int emin;                         // smallest exponent of the quantisation grid
+    int emin_floor;                   // lower bound of the finest grid exponent
     uint32_t max_nodes, n_prims;      // allocation bounds
 };
 
@@ -309,9 +402,9 @@ constexpr float kSahNode = 1.0f, kSahTri = XR_SAH_TRI;
 constexpr uint32_t kDecStride = 16;   // bytes per binary node: [0] leaf?, [1] j*, [i] split of i (2..8)
 
 __global__ void k_parents(uint32_t nint, const uint32_t* __restrict__ left, const uint32_t* __restrict__ right,
-                          uint32_t* __restrict__ parent_int, uint32_t* __restrict__ parent_leaf) {
+                          uint32_t* __restrict__ parent_int, uint32_t* __restrict__ parent_leaf, const uint32_t* made) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nint) return;
+    if (i >= nint || i >= *made) return;   // nodes a clustering without progress left out are not there
     const uint32_t lc = left[i], rc = right[i];
     if (lc & kLeafBit) parent_leaf[lc & ~kLeafBit] = i; else parent_int[lc] = i;
     if (rc & kLeafBit) parent_leaf[rc & ~kLeafBit] = i; else parent_int[rc] = i;
@@ -326,7 +419,10 @@ __device__ __forceinline__ void child_costs(uint32_t ref, const float* cost, con
         const float v = (dx * dy + dy * dz + dz * dx) * kSahTri;
         for (int i = 1; i <= 8; i++) c[i] = v;
     } else {
-        for (int i = 1; i <= 8; i++) c[i] = __ldcg(cost + 8u * ref + (i - 1));
+        const float4 a = __ldcg(reinterpret_cast<const float4*>(cost + 8u * (size_t)ref));
+        const float4 b = __ldcg(reinterpret_cast<const float4*>(cost + 8u * (size_t)ref) + 1);
+        c[1] = a.x; c[2] = a.y; c[3] = a.z; c[4] = a.w;
+        c[5] = b.x; c[6] = b.y; c[7] = b.z; c[8] = b.w;
     }
 }
 
@@ -347,34 +443,41 @@ __global__ void k_sah_dp(int n, const uint32_t* __restrict__ left, const uint32_
         child_costs(left[node], cost, sorted, tlo, thi, cl);
         child_costs(right[node], cost, sorted, tlo, thi, cr);
         float D[9];
-        uint8_t ks[9];
+        uint32_t ks[9];
+#pragma unroll
         for (int i = 2; i <= 8; i++) {
             D[i] = INFINITY;
-            ks[i] = 1;
+            ks[i] = 1u;
+#pragma unroll
             for (int k = 1; k < i; k++) {
                 const float v = cl[k] + cr[i - k];
-                if (v < D[i]) { D[i] = v; ks[i] = (uint8_t)k; }
+                if (v < D[i]) { D[i] = v; ks[i] = (uint32_t)k; }
             }
         }
-        int jstar = 2;
+        uint32_t jstar = 2u;
+        float dbest = D[2];
+#pragma unroll
         for (int i = 3; i <= 8; i++)
-            if (D[i] < D[jstar]) jstar = i;
+            if (D[i] < dbest) { dbest = D[i]; jstar = (uint32_t)i; }
         const float4 lo = __ldcg(nlo + node), hi = __ldcg(nhi + node);
         const float dx = hi.x - lo.x, dy = hi.y - lo.y, dz = hi.z - lo.z;
         const float A = dx * dy + dy * dz + dz * dx;
         const uint32_t cnt = count[node];
         const float c_leaf = cnt <= 3u ? A * kSahTri * (float)cnt : INFINITY;
-        const float c_int = A * kSahNode + D[jstar];
-        uint8_t* d = dec + (size_t)kDecStride * node;
-        float c = fminf(c_leaf, c_int);
-        d[0] = c_leaf <= c_int ? 1u : 0u;
-        d[1] = (uint8_t)jstar;
-        __stcg(cost + 8u * node, c);
+        const float c_int = A * kSahNode + dbest;
+        // 16 decision bytes and 8 costs, each written as whole words
+        uint32_t d[4] = {(c_leaf <= c_int ? 1u : 0u) | (jstar << 8), 0u, 0u, 0u};
+        float c[9];
+        c[1] = fminf(c_leaf, c_int);
+#pragma unroll
         for (int i = 2; i <= 8; i++) {
-            if (D[i] < c) { c = D[i]; d[i] = ks[i]; }
-            else d[i] = 0u;
-            __stcg(cost + 8u * node + (i - 1), c);
+            const bool less = D[i] < c[i - 1];
+            c[i] = less ? D[i] : c[i - 1];
+            if (less) d[i >> 2] |= ks[i] << (8 * (i & 3));
         }
+        *reinterpret_cast<uint4*>(dec + (size_t)kDecStride * node) = make_uint4(d[0], d[1], d[2], d[3]);
+        __stcg(reinterpret_cast<float4*>(cost + 8u * (size_t)node), make_float4(c[1], c[2], c[3], c[4]));
+        __stcg(reinterpret_cast<float4*>(cost + 8u * (size_t)node) + 1, make_float4(c[5], c[6], c[7], c[8]));
         node = parent_int[node];
     }
 }
@@ -413,135 +516,180 @@ __device__ __forceinline__ void pack_q(const uint8_t ql[3][8], const uint8_t qh[
     }
 }
 
-__global__ void k_collapse(CollapseArgs a) {
-    uint32_t task = blockIdx.x * blockDim.x + threadIdx.x;
-    if (task >= a.n_tasks) return;
-    const uint32_t bref = a.task_in[task];
-    const uint32_t widx = a.task_wide_in[task];
-    uint32_t refs[8];
-    int nc = 0;
-    if (bref & kLeafBit) {
-        refs[nc++] = bref;
-    } else if (a.dec) {
-        // the children the SAH decisions give: expand (node, slots) pairs depth first
-        uint32_t sx[8], si[8];
-        int ssp = 0;
-        sx[ssp] = bref; si[ssp] = a.dec[(size_t)kDecStride * bref + 1]; ssp++;
-        while (ssp > 0) {
-            ssp--;
-            const uint32_t x = sx[ssp], i = si[ssp];
-            if ((x & kLeafBit) || i <= 1u) {
-                if (nc < 8) refs[nc++] = x;
-                else atomicOr(&a.counters[3], 4u);
-                continue;
-            }
-            const uint32_t k = a.dec[(size_t)kDecStride * x + i];
-            if (k == 0u) { sx[ssp] = x; si[ssp] = i - 1u; ssp++; }
-            else if (ssp + 2 <= 8) {
-                sx[ssp] = a.right[x]; si[ssp] = i - k; ssp++;
-                sx[ssp] = a.left[x]; si[ssp] = k; ssp++;
-            } else {
-                atomicOr(&a.counters[3], 4u);
-            }
-        }
-    } else {
-        refs[nc++] = a.left[bref];
-        refs[nc++] = a.right[bref];
-        while (nc < 8) {
-            int best = -1;
-            float best_area = -1.0f;
-            for (int phase = 0; phase < 2 && best < 0; phase++) {
-                for (int c = 0; c < nc; c++) {
-                    uint32_t r = refs[c];
-                    if (r & kLeafBit) continue;
-                    uint32_t cnt = ref_count(r, a.count);
-                    if (phase == 0 ? cnt <= 3u : cnt > 3u) continue;
-                    float ar = half_area(a.nlo[r], a.nhi[r]);
-                    if (ar > best_area) { best_area = ar; best = c; }
+// Finest grid exponent: cells of at least 2^-17 of the largest coordinate.
+__host__ __device__ __forceinline__ int finest_exponent(float amax, int floor_e) {
+    int e;
+    frexpf(fmaxf(amax, 1e-20f), &e);
+    e -= 17;
+    return e > floor_e ? e : floor_e;
+}
+
+// One level of wide nodes, eight lanes per node, lane c holding child c (one thread per
+// node left each level waiting ~70 us on that thread's chain of loads, whatever its size:
+// 13 levels of the 1M-triangle scene took 0.96 ms, now 0.2).  The level's node count is read
+// on the device, so the host launches several levels without waiting for them.
+__global__ void __launch_bounds__(128) k_collapse(CollapseArgs a, uint32_t level) {
+    const uint32_t n_tasks = a.words->level_count[level];
+    const uint32_t c = threadIdx.x & 7u, g0 = threadIdx.x & 24u;   // child, first lane of the group
+    const uint32_t gm = 0xFFu << g0, upto = (2u << c) - 1u;
+    const int emin = finest_exponent(__uint_as_float(a.words->bounds[6]), a.emin_floor);
+    for (uint32_t task = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; task < n_tasks; task += (gridDim.x * blockDim.x) >> 3) {
+        const uint32_t bref = level ? a.task_in[task] : a.words->root;
+        const uint32_t widx = level ? a.task_wide_in[task] : 0u;
+        uint32_t ref = kInvalid;
+        if (bref & kLeafBit) {
+            if (c == 0u) ref = bref;
+        } else if (a.dec) {
+            // The children the SAH decisions give, left to right: lane c may hold a subtree x
+            // that takes the lanes c .. c + i - 1; splitting it sends its right part to lane
+            // c + k.
+            uint32_t x = bref, i = c == 0u ? a.dec[(size_t)kDecStride * bref + 1] : 0u;
+            while (true) {
+                const bool open = i > 1u && !(x & kLeafBit);
+                uint32_t k = 0u, r = 0u, l = 0u;
+                if (open) {
+                    k = a.dec[(size_t)kDecStride * x + i];
+                    l = a.left[x];
+                    r = a.right[x];
+                }
+                const uint32_t holders = (__ballot_sync(gm, i > 0u) >> g0) & 0xFFu;
+                if (!__any_sync(gm, open)) break;
+                const uint32_t from = 31u - __clz(holders & upto);   // lane 0 always holds one
+                const uint32_t fk = __shfl_sync(gm, k, g0 + from), fi = __shfl_sync(gm, i, g0 + from);
+                const uint32_t fr = __shfl_sync(gm, r, g0 + from);
+                if (open) {
+                    if (k) { x = l; i = k; }
+                    else i--;
+                } else if (i == 0u && fk && from + fk == c) {
+                    x = fr;
+                    i = fi - fk;
                 }
             }
-            if (best < 0) break;
-            uint32_t r = refs[best];
-            refs[best] = a.left[r];
-            refs[nc++] = a.right[r];
-        }
-    }
-    // boxes, parent box
-    float4 clo[8], chi[8];
-    float4 plo = make_float4(INFINITY, INFINITY, INFINITY, 0), phi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0);
-    for (int c = 0; c < nc; c++) {
-        ref_box(refs[c], a.nlo, a.nhi, a.tlo, a.thi, a.sorted, &clo[c], &chi[c]);
-        plo = make_float4(fminf(plo.x, clo[c].x), fminf(plo.y, clo[c].y), fminf(plo.z, clo[c].z), 0);
-        phi = make_float4(fmaxf(phi.x, chi[c].x), fmaxf(phi.y, chi[c].y), fmaxf(phi.z, chi[c].z), 0);
-    }
-    // slot assignment by octant of the child centre relative to the parent centre
-    int slot_of[8];
-    uint32_t used = 0;
-    float pcx = (plo.x + phi.x) * 0.5f, pcy = (plo.y + phi.y) * 0.5f, pcz = (plo.z + phi.z) * 0.5f;
-    uint32_t oct[8];
-    for (int c = 0; c < nc; c++) {
-        float cx = (clo[c].x + chi[c].x) * 0.5f, cy = (clo[c].y + chi[c].y) * 0.5f, cz = (clo[c].z + chi[c].z) * 0.5f;
-        oct[c] = (cx >= pcx ? 1u : 0u) | (cy >= pcy ? 2u : 0u) | (cz >= pcz ? 4u : 0u);
-        slot_of[c] = -1;
-        if (!(used & (1u << oct[c]))) { slot_of[c] = (int)oct[c]; used |= 1u << oct[c]; }
-    }
-    for (int c = 0; c < nc; c++) {
-        if (slot_of[c] >= 0) continue;
-        int best = -1, bd = 99;
-        for (int s = 0; s < 8; s++) {
-            if (used & (1u << s)) continue;
-            int dd = __popc((uint32_t)s ^ oct[c]);
-            if (dd < bd) { bd = dd; best = s; }
-        }
-        slot_of[c] = best;
-        used |= 1u << best;
-    }
-    // internal children and leaf triangle counts
-    uint32_t imask = 0, n_int = 0, n_tris = 0;
-    uint32_t cnt_of[8];
-    for (int c = 0; c < nc; c++) {
-        uint32_t cnt = ref_count(refs[c], a.count);
-        cnt_of[c] = cnt;
-        if (!(refs[c] & kLeafBit) && cnt > 3u) { imask |= 1u << slot_of[c]; n_int++; }
-        else n_tris += cnt;
-    }
-    uint32_t child_base = n_int ? atomicAdd(&a.counters[0], n_int) : 0u;
-    uint32_t tri_base = n_tris ? atomicAdd(&a.counters[1], n_tris) : 0u;
-    if (child_base + n_int > a.max_nodes || tri_base + n_tris > a.n_prims) {
-        atomicOr(&a.counters[3], 1u);   // inconsistent tree: reported by the host, nothing written
-        return;
-    }
-    WideNode nd;
-    int e[3];
-    float p3[3];
-    node_grid(plo, phi, a.emin, p3, e);
-    nd.px = p3[0]; nd.py = p3[1]; nd.pz = p3[2];
-    nd.exyz_imask = (uint32_t)(e[0] + 127) | ((uint32_t)(e[1] + 127) << 8) | ((uint32_t)(e[2] + 127) << 16) | (imask << 24);
-    nd.child_base = child_base;
-    nd.tri_base = tri_base;
-    uint8_t meta[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    uint8_t ql[3][8], qh[3][8];
-    for (int s = 0; s < 8; s++) for (int k = 0; k < 3; k++) { ql[k][s] = 0; qh[k][s] = 0; }
-    // leaf triangle offsets in slot order
-    uint32_t off = 0;
-    for (int s = 0; s < 8; s++) {
-        int c = -1;
-        for (int cc = 0; cc < nc; cc++) if (slot_of[cc] == s) c = cc;
-        if (c < 0) continue;
-        uint8_t cql[3], cqh[3];
-        child_q(clo[c], chi[c], p3, e, a.emin, cql, cqh);
-        for (int k = 0; k < 3; k++) { ql[k][s] = cql[k]; qh[k][s] = cqh[k]; }
-        uint32_t r = refs[c];
-        if (imask & (1u << s)) {
-            meta[s] = (uint8_t)(0x20u | (24u + (uint32_t)s));   // one bit, at 24 + slot
-            uint32_t rank = __popc(imask & ((1u << s) - 1u));
-            uint32_t slot = atomicAdd(&a.counters[2], 1u);
-            a.task_out[slot] = r;
-            a.task_wide_out[slot] = child_base + rank;
+            if (i) ref = x;
         } else {
+            // greedy widening, the same in every lane of the group
+            uint32_t refs[8];
+            int nc = 0;
+            refs[nc++] = a.left[bref];
+            refs[nc++] = a.right[bref];
+            while (nc < 8) {
+                int best = -1;
+                float best_area = -1.0f;
+                for (int phase = 0; phase < 2 && best < 0; phase++) {
+                    for (int j = 0; j < nc; j++) {
+                        uint32_t r = refs[j];
+                        if (r & kLeafBit) continue;
+                        uint32_t cnt = ref_count(r, a.count);
+                        if (phase == 0 ? cnt <= 3u : cnt > 3u) continue;
+                        float ar = half_area(a.nlo[r], a.nhi[r]);
+                        if (ar > best_area) { best_area = ar; best = j; }
+                    }
+                }
+                if (best < 0) break;
+                uint32_t r = refs[best];
+                refs[best] = a.left[r];
+                refs[nc++] = a.right[r];
+            }
+            if ((int)c < nc) ref = refs[c];
+        }
+        const bool there = ref != kInvalid;
+        // boxes, parent box
+        float4 lo = make_float4(INFINITY, INFINITY, INFINITY, 0), hi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0);
+        uint32_t cnt = 0u;
+        if (there) {
+            ref_box(ref, a.nlo, a.nhi, a.tlo, a.thi, a.sorted, &lo, &hi);
+            cnt = ref_count(ref, a.count);
+        }
+        float4 plo = lo, phi = hi;
+        for (int d = 1; d < 8; d <<= 1) {
+            plo = make_float4(fminf(plo.x, __shfl_xor_sync(gm, plo.x, d)), fminf(plo.y, __shfl_xor_sync(gm, plo.y, d)),
+                              fminf(plo.z, __shfl_xor_sync(gm, plo.z, d)), 0);
+            phi = make_float4(fmaxf(phi.x, __shfl_xor_sync(gm, phi.x, d)), fmaxf(phi.y, __shfl_xor_sync(gm, phi.y, d)),
+                              fmaxf(phi.z, __shfl_xor_sync(gm, phi.z, d)), 0);
+        }
+        // slot assignment by octant of the child centre relative to the parent centre: the
+        // first child of an octant takes it, each other one in turn the nearest free slot
+        const float pcx = (plo.x + phi.x) * 0.5f, pcy = (plo.y + phi.y) * 0.5f, pcz = (plo.z + phi.z) * 0.5f;
+        const float cx = (lo.x + hi.x) * 0.5f, cy = (lo.y + hi.y) * 0.5f, cz = (lo.z + hi.z) * 0.5f;
+        const uint32_t oct = (cx >= pcx ? 1u : 0u) | (cy >= pcy ? 2u : 0u) | (cz >= pcz ? 4u : 0u);
+        const uint32_t same = __match_any_sync(gm, there ? oct : 8u + c);
+        const bool first = there && (int)(g0 + c) == __ffs(same) - 1;
+        uint32_t slot = first ? oct : 8u;
+        uint32_t used = __reduce_or_sync(gm, first ? 1u << oct : 0u);
+        for (uint32_t rest = (__ballot_sync(gm, there && !first) >> g0) & 0xFFu; rest; rest &= rest - 1u) {
+            const uint32_t who = __ffs(rest) - 1u;
+            const uint32_t o = __shfl_sync(gm, oct, g0 + who);
+            uint32_t best = 0u;
+            int bd = 99;
+            for (uint32_t t = 0; t < 8u; t++) {
+                const int dd = __popc(t ^ o);
+                if (!((used >> t) & 1u) && dd < bd) { bd = dd; best = t; }
+            }
+            if (c == who) slot = best;
+            used |= 1u << best;
+        }
+        // internal children and leaf triangle counts
+        const bool internal = there && !(ref & kLeafBit) && cnt > 3u;
+        const bool leaf = there && !internal;
+        const uint32_t imask = __reduce_or_sync(gm, internal ? 1u << slot : 0u), n_int = __popc(imask);
+        const uint32_t n_tris = __reduce_add_sync(gm, leaf ? cnt : 0u);
+        uint32_t child_base = 0u, tri_base = 0u, task_base = 0u;
+        if (c == 0u) {
+            if (n_int) child_base = atomicAdd(&a.words->counters[0], n_int);
+            if (n_tris) tri_base = atomicAdd(&a.words->counters[1], n_tris);
+        }
+        child_base = __shfl_sync(gm, child_base, g0);
+        tri_base = __shfl_sync(gm, tri_base, g0);
+        if (child_base + n_int > a.max_nodes || tri_base + n_tris > a.n_prims) {
+            if (c == 0u) atomicOr(&a.words->counters[3], 1u);   // inconsistent tree: reported by the host, nothing written
+            continue;
+        }
+        if (c == 0u && n_int) task_base = atomicAdd(&a.words->level_count[level + 1u], n_int);
+        task_base = __shfl_sync(gm, task_base, g0);
+        int e[3];
+        float p3[3];
+        node_grid(plo, phi, emin, p3, e);
+        uint8_t ql[3] = {0, 0, 0}, qh[3] = {0, 0, 0};
+        if (there) child_q(lo, hi, p3, e, emin, ql, qh);
+        // leaf triangle offsets in slot order
+        uint32_t off = 0u;
+        for (uint32_t t = 0; t < 8u; t++) {
+            const uint32_t o = __shfl_sync(gm, leaf ? (slot << 8) | cnt : 0xFF00u, g0 + t);
+            if ((o >> 8) < slot) off += o & 0xFFu;
+        }
+        uint32_t meta = 0u;
+        if (internal) meta = 0x20u | (24u + slot);                      // one bit, at 24 + slot
+        else if (leaf) meta = (((1u << cnt) - 1u) << 5) | off;          // cnt bits, at the triangle offset
+        // the node: every lane's bytes at its slot
+        const uint32_t sh = 8u * (slot & 3u);
+        const bool w0 = there && slot < 4u, w1 = there && slot >= 4u;
+        uint32_t m[2], q[12];
+        m[0] = __reduce_or_sync(gm, w0 ? meta << sh : 0u);
+        m[1] = __reduce_or_sync(gm, w1 ? meta << sh : 0u);
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            q[2 * k] = __reduce_or_sync(gm, w0 ? (uint32_t)ql[k] << sh : 0u);
+            q[2 * k + 1] = __reduce_or_sync(gm, w1 ? (uint32_t)ql[k] << sh : 0u);
+            q[6 + 2 * k] = __reduce_or_sync(gm, w0 ? (uint32_t)qh[k] << sh : 0u);
+            q[6 + 2 * k + 1] = __reduce_or_sync(gm, w1 ? (uint32_t)qh[k] << sh : 0u);
+        }
+        uint4* dst = reinterpret_cast<uint4*>(a.nodes + widx);
+        if (c == 0u)
+            dst[0] = make_uint4(__float_as_uint(p3[0]), __float_as_uint(p3[1]), __float_as_uint(p3[2]),
+                                (uint32_t)(e[0] + 127) | ((uint32_t)(e[1] + 127) << 8) | ((uint32_t)(e[2] + 127) << 16) |
+                                    (imask << 24));
+        else if (c == 1u) dst[1] = make_uint4(child_base, tri_base, m[0], m[1]);
+        else if (c == 2u) dst[2] = make_uint4(q[0], q[1], q[2], q[3]);
+        else if (c == 3u) dst[3] = make_uint4(q[4], q[5], q[6], q[7]);
+        else if (c == 4u) dst[4] = make_uint4(q[8], q[9], q[10], q[11]);
+        if (internal) {
+            const uint32_t rank = __popc(imask & ((1u << slot) - 1u));
+            a.task_out[task_base + rank] = ref;
+            a.task_wide_out[task_base + rank] = child_base + rank;
+        } else if (leaf) {
             // the (at most 3) primitives of the subtree, left to right
             uint32_t prims[3], np = 0, dfs[4], dsp = 0;
-            dfs[dsp++] = r;
+            dfs[dsp++] = ref;
             while (dsp) {
                 uint32_t x = dfs[--dsp];
                 if (x & kLeafBit) {
@@ -552,31 +700,24 @@ __global__ void k_collapse(CollapseArgs a) {
                     dfs[dsp++] = a.left[x];
                 }
             }
-            uint32_t cnt = cnt_of[c];
-            if (np != cnt) { atomicOr(&a.counters[3], 2u); cnt = min(np, 3u); }
-            meta[s] = (uint8_t)((((1u << cnt) - 1u) << 5) | off);   // cnt bits, at the triangle offset
+            if (np != cnt) { atomicOr(&a.words->counters[3], 2u); cnt = min(np, 3u); }
             for (uint32_t j = 0; j < cnt; j++) {
                 uint32_t prim = prims[j];
                 if (a.records) {   // an instance record: world-to-object rows, {instance, root}
-                    float4* dst = a.tris + 4u * (tri_base + off + j);
-                    for (int w = 0; w < 4; w++) dst[w] = a.records[4u * prim + w];
+                    float4* rec = a.tris + 4u * (tri_base + off + j);
+                    for (int w = 0; w < 4; w++) rec[w] = a.records[4u * prim + w];
                     continue;
                 }
                 if (a.ref_prim) prim = a.ref_prim[prim];
                 uint4 id = a.tri_idx[prim];
                 float4 v0 = a.vpos[id.x], v1 = a.vpos[id.y], v2 = a.vpos[id.z];
-                float4* dst = a.tris + 3u * (tri_base + off + j);
-                dst[0] = make_float4(v0.x, v0.y, v0.z, __uint_as_float(prim));
-                dst[1] = make_float4(v1.x, v1.y, v1.z, 0.0f);
-                dst[2] = make_float4(v2.x, v2.y, v2.z, 0.0f);
+                float4* tri = a.tris + 3u * (tri_base + off + j);
+                tri[0] = make_float4(v0.x, v0.y, v0.z, __uint_as_float(prim));
+                tri[1] = make_float4(v1.x, v1.y, v1.z, 0.0f);
+                tri[2] = make_float4(v2.x, v2.y, v2.z, 0.0f);
             }
-            off += cnt;
         }
     }
-    nd.meta[0] = meta[0] | (meta[1] << 8) | (meta[2] << 16) | ((uint32_t)meta[3] << 24);
-    nd.meta[1] = meta[4] | (meta[5] << 8) | (meta[6] << 16) | ((uint32_t)meta[7] << 24);
-    pack_q(ql, qh, nd.q);
-    a.nodes[widx] = nd;
 }
 
 // ---- refit: new vertex positions under the same topology ----
@@ -765,82 +906,257 @@ __global__ void k_esc(const uint4* __restrict__ tri_idx, const float4* __restric
 #define XR_PLOC_RADIUS 64
 #endif
 constexpr int kPlocRadius = XR_PLOC_RADIUS;
-constexpr int kPlocBlock = 256;
+constexpr int kPlocBlock = 256;       // k_ploc_nn: two clusters per thread
+constexpr uint32_t kPlocWide = 1u << 16;   // up to this many: several lanes per cluster
+constexpr uint32_t kPlocTail = 2048;  // clusters that one block takes to the end
 
+// A cluster: {lo, reference}, {hi, primitives}.
 __global__ void k_ploc_init(uint32_t n, const uint32_t* __restrict__ sorted, const float4* __restrict__ tlo,
-                            const float4* __restrict__ thi, uint32_t* __restrict__ cref, float4* __restrict__ clo,
-                            float4* __restrict__ chi) {
+                            const float4* __restrict__ thi, float4* __restrict__ clo, float4* __restrict__ chi) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     uint32_t p = sorted[i];
-    cref[i] = i | kLeafBit;
-    clo[i] = tlo[p];
-    chi[i] = thi[p];
+    const float4 lo = tlo[p], hi = thi[p];
+    clo[i] = make_float4(lo.x, lo.y, lo.z, __uint_as_float(i | kLeafBit));
+    chi[i] = make_float4(hi.x, hi.y, hi.z, __uint_as_float(1u));
 }
 
-__global__ void __launch_bounds__(kPlocBlock) k_ploc_nn(uint32_t n, const float4* __restrict__ clo,
+__device__ __forceinline__ float merged_area(float4 alo, float4 ahi, float4 blo, float4 bhi) {
+    float dx = fmaxf(ahi.x, bhi.x) - fminf(alo.x, blo.x);
+    float dy = fmaxf(ahi.y, bhi.y) - fminf(alo.y, blo.y);
+    float dz = fmaxf(ahi.z, bhi.z) - fminf(alo.z, blo.z);
+    return dx * dy + dy * dz + dz * dx;
+}
+// What stands for a position outside the array: its merged area is infinite, so it never wins.
+__device__ __forceinline__ float4 nowhere(float s) { return make_float4(s * INFINITY, s * INFINITY, s * INFINITY, 0.0f); }
+
+// Nearest neighbours.  Candidates are taken in ascending order with a strict comparison:
+// of equal areas the lowest position wins, which orders pairs by area, lower index, upper
+// index.  A thread searches for two adjacent clusters, so that each candidate read from
+// shared memory serves two (reading it was the bound: 128 x 32 B per cluster); even and
+// odd positions are stored apart, so that the threads' reads are consecutive.  SPLIT > 1:
+// that many lanes share a pair's candidates, for counts that leave the chip idle and the
+// search a serial chain (2048 .. 64K clusters: 10.5 us a round with one lane, 5.5 with 8).
+template <int SPLIT>
+__global__ void __launch_bounds__(kPlocBlock) k_ploc_nn(const uint32_t* n_ptr, const float4* __restrict__ clo,
                                                         const float4* __restrict__ chi, uint32_t* __restrict__ nn) {
-    __shared__ float4 slo[kPlocBlock + 2 * kPlocRadius], shi[kPlocBlock + 2 * kPlocRadius];
-    const int base = (int)(blockIdx.x * kPlocBlock) - kPlocRadius;
-    for (int k = threadIdx.x; k < kPlocBlock + 2 * kPlocRadius; k += kPlocBlock) {
-        int j = base + k;
-        if (j >= 0 && j < (int)n) { slo[k] = clo[j]; shi[k] = chi[j]; }
+    constexpr int R = kPlocRadius, kPairs = kPlocBlock / SPLIT, kHalf = kPairs + R;
+    static_assert(R % 2 == 0, "even and odd candidates are stored apart");
+    __shared__ float4 slo[2][kHalf], shi[2][kHalf];
+    const int n = (int)*n_ptr;
+    const int first = (int)blockIdx.x * 2 * kPairs;
+    if (first >= n) return;
+    for (int k = threadIdx.x; k < 2 * kHalf; k += kPlocBlock) {
+        const int j = first - R + k;
+        const bool in = j >= 0 && j < n;
+        slo[k & 1][k >> 1] = in ? clo[j] : nowhere(-1.0f);
+        shi[k & 1][k >> 1] = in ? chi[j] : nowhere(1.0f);
     }
     __syncthreads();
-    const int i = (int)(blockIdx.x * kPlocBlock + threadIdx.x);
-    if (i >= (int)n) return;
-    const float4 alo = slo[threadIdx.x + kPlocRadius], ahi = shi[threadIdx.x + kPlocRadius];
-    float best = INFINITY;
-    int bj = -1;
-    for (int o = -kPlocRadius; o <= kPlocRadius; o++) {
-        int j = i + o;
-        if (o == 0 || j < 0 || j >= (int)n) continue;
-        float4 blo = slo[threadIdx.x + kPlocRadius + o], bhi = shi[threadIdx.x + kPlocRadius + o];
-        float dx = fmaxf(ahi.x, bhi.x) - fminf(alo.x, blo.x);
-        float dy = fmaxf(ahi.y, bhi.y) - fminf(alo.y, blo.y);
-        float dz = fmaxf(ahi.z, bhi.z) - fminf(alo.z, blo.z);
-        float a = dx * dy + dy * dz + dz * dx;
-        // total order on pairs: area, then the pair's lower index, then its upper index
-        bool better = a < best;
-        if (a == best && bj >= 0) {
-            int lo_new = min(i, j), hi_new = max(i, j), lo_old = min(i, bj), hi_old = max(i, bj);
-            better = lo_new < lo_old || (lo_new == lo_old && hi_new < hi_old);
+    const int t = threadIdx.x / SPLIT, i0 = first + 2 * t;
+    const float4 alo = slo[0][t + R / 2], ahi = shi[0][t + R / 2], blo = slo[1][t + R / 2], bhi = shi[1][t + R / 2];
+    float best0 = INFINITY, best1 = INFINITY;
+    int m0 = 2 * R + 2, m1 = 2 * R + 2;   // candidate's place: twice the step plus the parity (none: beyond the last)
+    // positions i0 - R .. i0 + R + 1: the first is out of the second cluster's reach, the
+    // last out of the first's, and neither is its own neighbour
+    auto step = [&](int m, bool e0, bool e1, bool o0, bool o1) {
+        const float4 elo = slo[0][t + m], ehi = shi[0][t + m];
+        if (e0) { const float a = merged_area(alo, ahi, elo, ehi); if (a < best0) { best0 = a; m0 = 2 * m; } }
+        if (e1) { const float a = merged_area(blo, bhi, elo, ehi); if (a < best1) { best1 = a; m1 = 2 * m; } }
+        const float4 olo = slo[1][min(t + m, kHalf - 1)], ohi = shi[1][min(t + m, kHalf - 1)];
+        if (o0) { const float a = merged_area(alo, ahi, olo, ohi); if (a < best0) { best0 = a; m0 = 2 * m + 1; } }
+        if (o1) { const float a = merged_area(blo, bhi, olo, ohi); if (a < best1) { best1 = a; m1 = 2 * m + 1; } }
+    };
+    if (SPLIT == 1) {
+        step(0, true, false, true, true);
+#pragma unroll 4
+        for (int m = 1; m < R / 2; m++) step(m, true, true, true, true);
+        step(R / 2, false, true, true, false);
+#pragma unroll 4
+        for (int m = R / 2 + 1; m < R; m++) step(m, true, true, true, true);
+        step(R, true, true, false, true);
+    } else {
+        for (int m = (int)threadIdx.x % SPLIT; m <= R; m += SPLIT) step(m, m != R / 2, m != 0, m != R, m != R / 2);
+#pragma unroll
+        for (int d = 1; d < SPLIT; d <<= 1) {
+            const float a0 = __shfl_xor_sync(0xFFFFFFFFu, best0, d), a1 = __shfl_xor_sync(0xFFFFFFFFu, best1, d);
+            const int p0 = __shfl_xor_sync(0xFFFFFFFFu, m0, d), p1 = __shfl_xor_sync(0xFFFFFFFFu, m1, d);
+            if (a0 < best0 || (a0 == best0 && p0 < m0)) { best0 = a0; m0 = p0; }
+            if (a1 < best1 || (a1 == best1 && p1 < m1)) { best1 = a1; m1 = p1; }
         }
-        if (better) { best = a; bj = j; }
+        if (threadIdx.x % SPLIT) return;
     }
-    nn[i] = bj < 0 ? (uint32_t)i : (uint32_t)bj;
+    if (i0 < n) nn[i0] = (uint32_t)(m0 > 2 * R + 1 ? i0 : i0 - R + m0);
+    if (i0 + 1 < n) nn[i0 + 1] = (uint32_t)(m1 > 2 * R + 1 ? i0 + 1 : i0 - R + m1);
 }
 
-__global__ void k_ploc_merge(uint32_t n, const uint32_t* __restrict__ nn, const uint32_t* __restrict__ cref,
-                             const float4* __restrict__ clo, const float4* __restrict__ chi, uint32_t* __restrict__ tref,
-                             float4* __restrict__ tlo, float4* __restrict__ thi, uint32_t* __restrict__ keep,
-                             uint32_t* __restrict__ left, uint32_t* __restrict__ right, uint32_t* __restrict__ count,
-                             float4* __restrict__ nlo, float4* __restrict__ nhi, uint32_t* node_counter, uint32_t max_nodes) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t j = nn[i];
-    const bool mutual = j != i && nn[j] == i;
-    if (mutual && i > j) { keep[i] = 0u; return; }   // merged into position j
-    keep[i] = 1u;
-    if (!mutual) { tref[i] = cref[i]; tlo[i] = clo[i]; thi[i] = chi[i]; return; }
-    const uint32_t k = atomicAdd(node_counter, 1u);
-    const float4 al = clo[i], ah = chi[i], bl = clo[j], bh = chi[j];
-    const float4 ml = make_float4(fminf(al.x, bl.x), fminf(al.y, bl.y), fminf(al.z, bl.z), 0.0f);
-    const float4 mh = make_float4(fmaxf(ah.x, bh.x), fmaxf(ah.y, bh.y), fmaxf(ah.z, bh.z), 0.0f);
-    const uint32_t ra = cref[i], rb = cref[j];
-    if (k < max_nodes) {
-        left[k] = ra;
-        right[k] = rb;
-        count[k] = ((ra & kLeafBit) ? 1u : count[ra]) + ((rb & kLeafBit) ? 1u : count[rb]);
-        nlo[k] = ml;
-        nhi[k] = mh;
+struct PlocTree {   // the binary tree being made
+    uint32_t* left; uint32_t* right; uint32_t* count;
+    float4* nlo; float4* nhi;
+    uint32_t max_nodes;
+};
+// Node k over two clusters; returns the merged cluster in alo, ahi.
+__device__ __forceinline__ void ploc_node(const PlocTree& T, uint32_t k, float4& alo, float4& ahi, float4 blo, float4 bhi) {
+    const uint32_t cnt = __float_as_uint(ahi.w) + __float_as_uint(bhi.w);
+    if (k < T.max_nodes) {
+        T.left[k] = __float_as_uint(alo.w);
+        T.right[k] = __float_as_uint(blo.w);
+        T.count[k] = cnt;
     }
-    tref[i] = k;
-    tlo[i] = ml;
-    thi[i] = mh;
+    alo = make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), __uint_as_float(k));
+    ahi = make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), __uint_as_float(cnt));
+    if (k < T.max_nodes) {
+        T.nlo[k] = make_float4(alo.x, alo.y, alo.z, 0.0f);
+        T.nhi[k] = make_float4(ahi.x, ahi.y, ahi.z, 0.0f);
+    }
 }
 
-// exclusive scan of keep[] in blocks of 1024 (block sums to `sums`)
+// Merges the mutual pairs of 1024 positions; the clusters that stay go to the start of the
+// block's 1024 places of (olo, ohi), in order, and their number to sums[block].
+__global__ void __launch_bounds__(1024) k_ploc_merge(const uint32_t* n_ptr, const uint32_t* __restrict__ nn,
+                                                     const float4* __restrict__ clo, const float4* __restrict__ chi,
+                                                     float4* __restrict__ olo, float4* __restrict__ ohi,
+                                                     uint32_t* __restrict__ sums, uint32_t* made, PlocTree T) {
+    __shared__ uint32_t wsum[32];
+    const uint32_t n = *n_ptr, i = blockIdx.x * 1024u + threadIdx.x, lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    if (blockIdx.x * 1024u >= n) return;
+    bool keep = false;
+    float4 lo, hi;
+    if (i < n) {
+        const uint32_t j = n > 1u ? nn[i] : i;
+        const bool mutual = j != i && nn[j] == i;
+        keep = !(mutual && i > j);   // else merged into position j
+        if (keep) {
+            lo = clo[i];
+            hi = chi[i];
+            if (mutual) ploc_node(T, atomicAdd(made, 1u), lo, hi, clo[j], chi[j]);
+        }
+    }
+    const uint32_t kept = __ballot_sync(0xFFFFFFFFu, keep);
+    if (lane == 0u) wsum[w] = __popc(kept);
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+    for (uint32_t v = 0; v < 32u; v++) {
+        if (v < w) before += wsum[v];
+        all += wsum[v];
+    }
+    if (keep) {
+        const uint32_t at = blockIdx.x * 1024u + before + __popc(kept & ((1u << lane) - 1u));
+        olo[at] = lo;
+        ohi[at] = hi;
+    }
+    if (threadIdx.x == 0u) sums[blockIdx.x] = all;
+}
+
+// Closes the gaps between the blocks' clusters; each block adds up the counts before its own.
+__global__ void __launch_bounds__(256) k_ploc_compact(const uint32_t* n_ptr, uint32_t* n_next,
+                                                      const uint32_t* __restrict__ sums, const float4* __restrict__ olo,
+                                                      const float4* __restrict__ ohi, float4* __restrict__ clo,
+                                                      float4* __restrict__ chi) {
+    __shared__ uint32_t wsum[8];
+    const uint32_t nb = (*n_ptr + 1023u) / 1024u, b = blockIdx.x;
+    if (b >= nb) return;
+    uint32_t s = 0;
+    for (uint32_t i = threadIdx.x; i < b; i += 256u) s += sums[i];
+    s = __reduce_add_sync(0xFFFFFFFFu, s);
+    if ((threadIdx.x & 31u) == 0u) wsum[threadIdx.x >> 5] = s;
+    __syncthreads();
+    uint32_t before = 0;
+    for (int w = 0; w < 8; w++) before += wsum[w];
+    const uint32_t cnt = sums[b];
+    for (uint32_t i = threadIdx.x; i < cnt; i += 256u) {
+        clo[before + i] = olo[b * 1024u + i];
+        chi[before + i] = ohi[b * 1024u + i];
+    }
+    if (b == nb - 1u && threadIdx.x == 0u) *n_next = before + cnt;
+}
+
+// The last rounds, from at most kPlocTail clusters to one, in one block: at 1M primitives
+// 45 of the 75 rounds have fewer, and three launches each would cost more than their work.
+// As clusters get fewer, more lanes share the search of one.
+constexpr size_t kPlocTailSmem = kPlocTail * (2 * sizeof(float4) + sizeof(uint32_t));
+__global__ void __launch_bounds__(1024) k_ploc_tail(uint32_t* n_ptr, const float4* __restrict__ clo,
+                                                    const float4* __restrict__ chi, BuildWords* words, PlocTree T) {
+    extern __shared__ float4 tail_mem[];
+    float4 *lo = tail_mem, *hi = tail_mem + kPlocTail;
+    uint32_t* nn = reinterpret_cast<uint32_t*>(tail_mem + 2 * kPlocTail);
+    __shared__ uint32_t wsum[32], made;
+    const uint32_t t = threadIdx.x, lane = t & 31u, w = t >> 5;
+    uint32_t n = *n_ptr;
+    if (n > kPlocTail) return;   // not the host's promise: `made` will not match
+    for (uint32_t i = t; i < n; i += 1024u) { lo[i] = clo[i]; hi[i] = chi[i]; }
+    if (t == 0u) made = words->made;
+    __syncthreads();
+    while (n > 1u) {
+        uint32_t share = 1u;   // lanes per cluster
+        while (share < 32u && n * share * 2u <= 1024u) share <<= 1;
+        const uint32_t sub = t & (share - 1u);
+        for (uint32_t base = 0; base < n; base += 1024u / share) {
+            const uint32_t c = base + t / share;
+            float best = INFINITY;
+            uint32_t bj = kInvalid;
+            if (c < n) {
+                const float4 alo = lo[c], ahi = hi[c];
+                const int end = min((int)c + kPlocRadius, (int)n - 1);
+                int j = (int)c - kPlocRadius + (int)sub;
+                if (j < 0) j += (-j + (int)share - 1) / (int)share * (int)share;
+                for (; j <= end; j += (int)share) {
+                    const float a = merged_area(alo, ahi, lo[j], hi[j]);
+                    if (a < best && j != (int)c) { best = a; bj = (uint32_t)j; }
+                }
+            }
+            for (uint32_t d = 1; d < share; d <<= 1) {
+                const float oa = __shfl_xor_sync(0xFFFFFFFFu, best, d);
+                const uint32_t oj = __shfl_xor_sync(0xFFFFFFFFu, bj, d);
+                if (oa < best || (oa == best && oj < bj)) { best = oa; bj = oj; }
+            }
+            if (c < n && sub == 0u) nn[c] = bj == kInvalid ? c : bj;
+        }
+        __syncthreads();
+        // merge and close the gaps, 1024 positions at a time: writes go at or before the
+        // positions read in the same step, after all of its reads
+        uint32_t out = 0u;
+        for (uint32_t base = 0; base < n; base += 1024u) {
+            const uint32_t i = base + t;
+            bool keep = false;
+            float4 al, ah;
+            if (i < n) {
+                const uint32_t j = nn[i];
+                const bool mutual = j != i && nn[j] == i;
+                keep = !(mutual && i > j);
+                if (keep) {
+                    al = lo[i];
+                    ah = hi[i];
+                    if (mutual) ploc_node(T, atomicAdd(&made, 1u), al, ah, lo[j], hi[j]);
+                }
+            }
+            const uint32_t kept = __ballot_sync(0xFFFFFFFFu, keep);
+            if (lane == 0u) wsum[w] = __popc(kept);
+            __syncthreads();
+            uint32_t before = 0, all = 0;
+            for (uint32_t v = 0; v < 32u; v++) {
+                if (v < w) before += wsum[v];
+                all += wsum[v];
+            }
+            if (keep) {
+                const uint32_t at = out + before + __popc(kept & ((1u << lane) - 1u));
+                lo[at] = al;
+                hi[at] = ah;
+            }
+            out += all;
+            __syncthreads();
+        }
+        if (out == n) break;   // no progress (infinite areas): `made` will not match
+        n = out;
+    }
+    if (t == 0u) {
+        words->made = made;
+        words->root = __float_as_uint(lo[0].w);
+        *n_ptr = n;
+    }
+}
+
+// exclusive scan in blocks of 1024 (block sums to `sums`)
 __global__ void __launch_bounds__(1024) k_scan_local(const uint32_t* __restrict__ in, uint32_t n,
                                                      uint32_t* __restrict__ out, uint32_t* __restrict__ sums) {
     __shared__ uint32_t warp_sums[32];
@@ -875,18 +1191,6 @@ __global__ void k_scan_top(uint32_t* sums, uint32_t nb) {
     sums[nb] = acc;
 }
 
-__global__ void k_ploc_compact(uint32_t n, const uint32_t* __restrict__ keep, const uint32_t* __restrict__ pos,
-                               const uint32_t* __restrict__ sums, const uint32_t* __restrict__ tref,
-                               const float4* __restrict__ tlo, const float4* __restrict__ thi,
-                               uint32_t* __restrict__ cref, float4* __restrict__ clo, float4* __restrict__ chi) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || !keep[i]) return;
-    uint32_t d = pos[i] + sums[i / 1024u];
-    cref[d] = tref[i];
-    clo[d] = tlo[i];
-    chi[d] = thi[i];
-}
-
 template <typename T>
 xr_status dalloc(Context* ctx, T** p, size_t count) {
     return cuda_check(ctx, cudaMalloc((void**)p, std::max<size_t>(count, 1) * sizeof(T)), "cudaMalloc (bvh)");
@@ -918,169 +1222,164 @@ xr_status build_wide(Context* ctx, WideBuild& B) {
 
     float4 *tlo = nullptr, *thi = nullptr, *nlo = nullptr, *nhi = nullptr;
     uint64_t *k0 = nullptr, *k1 = nullptr;
-    uint32_t *v0 = nullptr, *v1 = nullptr, *bounds = nullptr, *hist = nullptr;
+    uint32_t *v0 = nullptr, *v1 = nullptr, *hist = nullptr;
     uint32_t *left = nullptr, *right = nullptr, *pint = nullptr, *pleaf = nullptr, *flags = nullptr;
     uint32_t* range = nullptr;   // primitives below each binary internal node
-    uint32_t *ta = nullptr, *tb = nullptr, *wa = nullptr, *wb = nullptr, *counters = nullptr;
+    uint32_t *ta = nullptr, *tb = nullptr, *wa = nullptr, *wb = nullptr;
+    BuildWords* words = nullptr;
     WideNode* nodes_tmp = nullptr;
     float* sah_cost = nullptr;     // SAH collapse: 8 costs and kDecStride decision bytes per binary node
     uint8_t* sah_dec = nullptr;
     uint32_t* sah_flags = nullptr;
+    // clustering: clusters, their next round's, nearest neighbours, block counts
+    float4 *clo = nullptr, *chi = nullptr, *olo = nullptr, *ohi = nullptr;
+    uint32_t *nn = nullptr, *sums = nullptr;
+    void* scratch = nullptr;
+    BuildWords back;
     xr_status s = XR_OK;
     const uint32_t nint = n > 1 ? n - 1 : 1;
-    const uint32_t chunk = 4096;
+    const uint32_t chunk = 1024;   // keys per sort block: 4096 left a third of the chip idle at 1M (54 + 28 + 11 us a pass with one block scanning, now 5 + 19 + 6)
     const uint32_t nblk = (n + chunk - 1) / chunk;
-    if ((s = salloc(ctx, &tlo, n)) || (s = salloc(ctx, &thi, n)) || (s = salloc(ctx, &k0, n)) ||
-        (s = salloc(ctx, &k1, n)) || (s = salloc(ctx, &v0, n)) || (s = salloc(ctx, &v1, n)) ||
-        (s = salloc(ctx, &bounds, 8)) || (s = salloc(ctx, &hist, 256 * nblk)) || (s = salloc(ctx, &left, nint)) ||
-        (s = salloc(ctx, &right, nint)) || (s = salloc(ctx, &pint, nint)) || (s = salloc(ctx, &pleaf, n)) ||
-        (s = salloc(ctx, &flags, nint + 1)) || (s = salloc(ctx, &range, nint)) || (s = salloc(ctx, &nlo, nint)) ||
-        (s = salloc(ctx, &nhi, nint)) || (s = salloc(ctx, &ta, n)) || (s = salloc(ctx, &tb, n)) ||
-        (s = salloc(ctx, &wa, n)) || (s = salloc(ctx, &wb, n)) || (s = salloc(ctx, &counters, 4)) ||
-        (s = salloc(ctx, &nodes_tmp, nint)) ||
-        (!B.slots_into && (s = dalloc(ctx, &B.slots, (size_t)slot_words * n))))
-        goto done;
+    const char* builder = getenv("XR_BVH_BUILDER");
+    const bool use_lbvh = B.builder == 2 || (B.builder == 0 && builder && strcmp(builder, "lbvh") == 0);
+    const bool ploc = n > 1 && !use_lbvh;
+    const char* coll = getenv("XR_BVH_COLLAPSE");   // greedy: the area-greedy widening instead of the SAH decisions
+    const bool sah = n > 1 && !(coll && strcmp(coll, "greedy") == 0);
+    const uint32_t np = ploc ? n : 0u, nd = sah ? nint : 0u;
+    {   // one stream-ordered allocation holds all scratch
+        struct Item { void** dst; size_t bytes; };
+        std::vector<Item> items;
+        auto add = [&](auto** dst, size_t count) { items.push_back({(void**)dst, count * sizeof(**dst)}); };
+        add(&tlo, n); add(&thi, n); add(&k0, n); add(&k1, n); add(&v0, n); add(&v1, n);
+        add(&hist, 256 * ((size_t)nblk + 1)); add(&left, nint); add(&right, nint); add(&pint, nint); add(&pleaf, n);
+        add(&flags, (size_t)nint + 1); add(&range, nint); add(&nlo, nint); add(&nhi, nint);
+        add(&ta, n); add(&tb, n); add(&wa, n); add(&wb, n); add(&words, 1); add(&nodes_tmp, nint);
+        add(&clo, np); add(&chi, np); add(&olo, np); add(&ohi, np); add(&nn, np); add(&sums, np / 1024 + 1);
+        add(&sah_cost, 8 * (size_t)nd); add(&sah_dec, kDecStride * (size_t)nd); add(&sah_flags, (size_t)nd + 1);
+        auto up = [](size_t v) { return (v + 255u) & ~size_t(255u); };
+        size_t total = 0;
+        for (const Item& it : items) total += up(it.bytes);
+        if ((s = pool_alloc_bytes(ctx, &scratch, total, "bvh scratch"))) goto done;
+        size_t off = 0;
+        for (const Item& it : items) { *it.dst = (char*)scratch + off; off += up(it.bytes); }
+    }
+    if (!B.slots_into && (s = dalloc(ctx, &B.slots, (size_t)slot_words * n))) goto done;
     if (B.slots_into) B.slots = B.slots_into;
     {
-        uint32_t binit[8] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u, 0u, 0u};
-        cudaMemcpyAsync(bounds, binit, sizeof(binit), cudaMemcpyHostToDevice, st);
-        uint32_t blocks = (n + 255) / 256;
-        k_tri_prep<<<blocks, 256, 0, st>>>(B.tri_idx, B.vpos, n, B.box_lo, B.box_hi, tlo, thi, bounds);
-        k_morton<<<blocks, 256, 0, st>>>(tlo, thi, n, bounds, k0, v0);
-        for (int pass = 0; pass < 8; pass++) {
-            int shift = pass * 8;
-            k_sort_hist<<<nblk, 256, 0, st>>>(k0, n, chunk, shift, hist, nblk);
-            k_sort_scan<<<1, 1024, 0, st>>>(hist, 256 * nblk);
-            k_sort_scatter<<<nblk, kSortThreads, 0, st>>>(k0, v0, k1, v1, n, chunk, shift, hist, nblk);
-            std::swap(k0, k1);
-            std::swap(v0, v1);
+        const uint32_t blocks = (n + 255) / 256;
+        k_build_init<<<1, 256, 0, st>>>(words, n, n == 1 ? kLeafBit : 0u);
+        k_tri_prep<<<std::min<uint32_t>((n + kPrepBlock - 1) / kPrepBlock, 4u * (uint32_t)ctx->sm_count), kPrepBlock, 0, st>>>(
+            B.tri_idx, B.vpos, n, B.box_lo, B.box_hi, tlo, thi, words->bounds);
+        k_morton<<<blocks, 256, 0, st>>>(tlo, thi, n, words->bounds, k0, v0);
+        if (n <= kSmallSort) {
+            k_sort_small<<<1, 1024, 0, st>>>(k0, v0, n);
+        } else {
+            uint32_t* tot = hist + 256 * (size_t)nblk;
+            for (int pass = 0; pass < 8; pass++) {
+                int shift = pass * 8;
+                k_sort_hist<<<nblk, 256, 0, st>>>(k0, n, chunk, shift, hist, nblk);
+                k_sort_rows<<<256, kSortThreads, 0, st>>>(hist, tot, nblk);
+                k_sort_scatter<<<nblk, kSortThreads, 0, st>>>(k0, v0, k1, v1, n, chunk, shift, hist, tot, nblk);
+                std::swap(k0, k1);
+                std::swap(v0, v1);
+            }
         }
-        uint32_t bh[8];
-        cudaMemcpyAsync(bh, bounds, sizeof(bh), cudaMemcpyDeviceToHost, st);
-        if ((s = cuda_check(ctx, cudaStreamSynchronize(st), "bvh: sort"))) goto done;
-        float amax;
-        memcpy(&amax, &bh[6], 4);
-        int emin;
-        frexpf(fmaxf(amax, 1e-20f), &emin);
-        emin -= 17;   // cells of at least 2^-17 of the largest coordinate
-        emin = std::max(emin, B.emin_floor);
-        B.emin = emin;
         cudaMemsetAsync(pint, 0xFF, nint * 4, st);
         cudaMemsetAsync(pleaf, 0xFF, (size_t)n * 4, st);
         cudaMemsetAsync(flags, 0, (nint + 1) * 4, st);
-        uint32_t root_ref = 0u;
-        const char* builder = getenv("XR_BVH_BUILDER");
-        const bool use_lbvh = B.builder == 2 || (B.builder == 0 && builder && strcmp(builder, "lbvh") == 0);
-        if (n == 1) {
-            root_ref = 0u | kLeafBit;
-        } else if (use_lbvh) {
+        if (n > 1 && use_lbvh) {
             k_karras<<<(n - 1 + 255) / 256, 256, 0, st>>>(k0, (int)n, left, right, pint, pleaf, range);
-            k_bounds<<<(n + 255) / 256, 256, 0, st>>>((int)n, left, right, pint, pleaf, v0, tlo, thi, nlo, nhi, flags);
-        } else {
-            // PLOC rounds; the ping-pong cluster arrays reuse the Morton key buffers' space
-            uint32_t *cref0 = nullptr, *cref1 = nullptr, *nnb = nullptr, *keep = nullptr, *pos = nullptr, *sums = nullptr;
-            float4 *clo0 = nullptr, *chi0 = nullptr, *clo1 = nullptr, *chi1 = nullptr;
-            const uint32_t nbmax = (n + 1023) / 1024;
-            if ((s = salloc(ctx, &cref0, n)) || (s = salloc(ctx, &cref1, n)) || (s = salloc(ctx, &nnb, n)) ||
-                (s = salloc(ctx, &keep, n)) || (s = salloc(ctx, &pos, n)) || (s = salloc(ctx, &sums, nbmax + 1)) ||
-                (s = salloc(ctx, &clo0, n)) || (s = salloc(ctx, &chi0, n)) || (s = salloc(ctx, &clo1, n)) ||
-                (s = salloc(ctx, &chi1, n))) {
-                sfree(ctx, cref0); sfree(ctx, cref1); sfree(ctx, nnb); sfree(ctx, keep); sfree(ctx, pos); sfree(ctx, sums);
-                sfree(ctx, clo0); sfree(ctx, chi0); sfree(ctx, clo1); sfree(ctx, chi1);
-                goto done;
-            }
-            cudaMemsetAsync(counters + 3, 0, 4, st);
-            k_ploc_init<<<(n + 255) / 256, 256, 0, st>>>(n, v0, tlo, thi, cref0, clo0, chi0);
-            uint32_t cnt = n, rounds = 0;
-            while (cnt > 1 && !s) {
-                const uint32_t nb = (cnt + 1023) / 1024;
-                k_ploc_nn<<<(cnt + kPlocBlock - 1) / kPlocBlock, kPlocBlock, 0, st>>>(cnt, clo0, chi0, nnb);
-                k_ploc_merge<<<(cnt + 255) / 256, 256, 0, st>>>(cnt, nnb, cref0, clo0, chi0, cref1, clo1, chi1, keep,
-                                                                 left, right, range, nlo, nhi, counters + 3, nint);
-                k_scan_local<<<nb, 1024, 0, st>>>(keep, cnt, pos, sums);
-                k_scan_top<<<1, 32, 0, st>>>(sums, nb);
-                k_ploc_compact<<<(cnt + 255) / 256, 256, 0, st>>>(cnt, keep, pos, sums, cref1, clo1, chi1, cref0, clo0, chi0);
-                uint32_t next = 0;
-                cudaMemcpyAsync(&next, sums + nb, 4, cudaMemcpyDeviceToHost, st);
+            k_bounds<<<blocks, 256, 0, st>>>((int)n, left, right, pint, pleaf, v0, tlo, thi, nlo, nhi, flags);
+        } else if (ploc) {
+            const PlocTree T{left, right, range, nlo, nhi, nint};
+            k_ploc_init<<<blocks, 256, 0, st>>>(n, v0, tlo, thi, clo, chi);
+            // Rounds until one block can take the rest.  The kernels read the cluster count on
+            // the device, so the host sends several rounds (a round keeps about five sixths)
+            // with the count of the batch's start and waits once per batch.
+            uint32_t cnt = n, side = 0;
+            while (cnt > kPlocTail && !s) {
+                uint32_t rounds = 1;
+                for (uint32_t c = cnt; c > kPlocTail && rounds < 8; c -= c / 6) rounds++;
+                for (uint32_t r = 0; r < rounds; r++, side ^= 1u) {
+                    uint32_t *cur = &words->clusters[side], *next = &words->clusters[side ^ 1u];
+                    if (cnt > kPlocWide)
+                        k_ploc_nn<1><<<(cnt + 2 * kPlocBlock - 1) / (2 * kPlocBlock), kPlocBlock, 0, st>>>(cur, clo, chi, nn);
+                    else
+                        k_ploc_nn<8><<<(cnt + kPlocBlock / 4 - 1) / (kPlocBlock / 4), kPlocBlock, 0, st>>>(cur, clo, chi, nn);
+                    k_ploc_merge<<<(cnt + 1023) / 1024, 1024, 0, st>>>(cur, nn, clo, chi, olo, ohi, sums, &words->made, T);
+                    k_ploc_compact<<<(cnt + 1023) / 1024, 256, 0, st>>>(cur, next, sums, olo, ohi, clo, chi);
+                }
+                uint32_t left_over = 0;
+                cudaMemcpyAsync(&left_over, &words->clusters[side], 4, cudaMemcpyDeviceToHost, st);
                 if ((s = cuda_check(ctx, cudaStreamSynchronize(st), "bvh: ploc"))) break;
-                if (next >= cnt || ++rounds > 100000) { s = fail(ctx, XR_ERR_STATE, "bvh: clustering made no progress"); break; }
-                cnt = next;
+                if (left_over >= cnt) s = fail(ctx, XR_ERR_STATE, "bvh: clustering made no progress");
+                cnt = left_over;
             }
-            uint32_t made = 0;
-            if (!s) {
-                cudaMemcpy(&root_ref, cref0, 4, cudaMemcpyDeviceToHost);
-                cudaMemcpy(&made, counters + 3, 4, cudaMemcpyDeviceToHost);
-                if (made != n - 1) s = fail(ctx, XR_ERR_STATE, "bvh: clustering built the wrong number of nodes");
-            }
-            sfree(ctx, cref0); sfree(ctx, cref1); sfree(ctx, nnb); sfree(ctx, keep); sfree(ctx, pos); sfree(ctx, sums);
-            sfree(ctx, clo0); sfree(ctx, chi0); sfree(ctx, clo1); sfree(ctx, chi1);
             if (s) goto done;
+            if ((s = cuda_check(ctx, cudaFuncSetAttribute(k_ploc_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                          (int)kPlocTailSmem), "bvh: ploc"))) goto done;
+            k_ploc_tail<<<1, 1024, kPlocTailSmem, st>>>(&words->clusters[side], clo, chi, words, T);
         }
-        // SAH decisions for the collapse (XR_BVH_COLLAPSE=greedy: the area-greedy widening)
-        const char* coll = getenv("XR_BVH_COLLAPSE");
-        const bool sah = n > 1 && !(coll && strcmp(coll, "greedy") == 0);
+        cudaMemsetAsync(sah_flags, 0, (nd + 1) * 4, st);
         if (sah) {
-            if ((s = salloc(ctx, &sah_cost, 8 * (size_t)nint)) || (s = salloc(ctx, &sah_dec, kDecStride * (size_t)nint)) ||
-                (s = salloc(ctx, &sah_flags, nint + 1)))
-                goto done;
-            if (!use_lbvh) k_parents<<<(nint + 255) / 256, 256, 0, st>>>(nint, left, right, pint, pleaf);
-            cudaMemsetAsync(sah_flags, 0, (nint + 1) * 4, st);
-            k_sah_dp<<<(n + 255) / 256, 256, 0, st>>>((int)n, left, right, range, pint, pleaf, v0, tlo, thi, nlo, nhi,
-                                                      sah_cost, sah_dec, sah_flags);
+            if (!use_lbvh) k_parents<<<(nint + 255) / 256, 256, 0, st>>>(nint, left, right, pint, pleaf, &words->made);
+            k_sah_dp<<<blocks, 256, 0, st>>>((int)n, left, right, range, pint, pleaf, v0, tlo, thi, nlo, nhi, sah_cost,
+                                             sah_dec, sah_flags);
         }
-        uint32_t cinit[4] = {1u, 0u, 0u, 0u};
-        cudaMemcpyAsync(counters, cinit, sizeof(cinit), cudaMemcpyHostToDevice, st);
-        uint32_t zero = 0u;
-        cudaMemcpyAsync(ta, &root_ref, 4, cudaMemcpyHostToDevice, st);
-        cudaMemcpyAsync(wa, &zero, 4, cudaMemcpyHostToDevice, st);
-        uint32_t ntask = 1, depth = 0;
-        B.level_off.push_back(0u);
-        B.level_off.push_back(1u);   // level 0: the root
-        while (ntask > 0) {
-            CollapseArgs ca;
-            ca.left = left; ca.right = right; ca.count = range; ca.nlo = nlo; ca.nhi = nhi; ca.tlo = tlo; ca.thi = thi;
-            ca.sorted = v0; ca.tri_idx = B.tri_idx; ca.vpos = B.vpos; ca.records = B.records;
-            ca.dec = sah ? sah_dec : nullptr;
-            ca.ref_prim = B.ref_prim;
-            ca.task_in = ta; ca.task_wide_in = wa; ca.n_tasks = ntask; ca.task_out = tb; ca.task_wide_out = wb;
-            ca.counters = counters; ca.nodes = nodes_tmp; ca.tris = B.slots; ca.emin = emin;
-            ca.max_nodes = nint; ca.n_prims = n;
-            cudaMemsetAsync(counters + 2, 0, 4, st);
-            k_collapse<<<(ntask + 127) / 128, 128, 0, st>>>(ca);
-            uint32_t cnt3[3];
-            cudaMemcpyAsync(cnt3, counters, sizeof(cnt3), cudaMemcpyDeviceToHost, st);
+        CollapseArgs ca;
+        ca.left = left; ca.right = right; ca.count = range; ca.nlo = nlo; ca.nhi = nhi; ca.tlo = tlo; ca.thi = thi;
+        ca.sorted = v0; ca.tri_idx = B.tri_idx; ca.vpos = B.vpos; ca.records = B.records;
+        ca.dec = sah ? sah_dec : nullptr;
+        ca.ref_prim = B.ref_prim;
+        ca.words = words; ca.nodes = nodes_tmp; ca.tris = B.slots; ca.emin_floor = B.emin_floor;
+        ca.max_nodes = nint; ca.n_prims = n;
+        // Levels in batches: enough for a well-filled tree and a few more, then eight at a time.
+        uint32_t level = 0, until = 5;
+        for (uint32_t c = n; c > 1; c /= 8) until++;
+        uint32_t bflag = 0, dflag = 0;
+        while (true) {
+            for (; level < until; level++) {
+                // a level has at most 8 times the nodes of the one above
+                const uint64_t most = level < 8 ? std::min<uint64_t>(1ull << (3 * level), nint) : nint;
+                const uint32_t grid = (uint32_t)std::min<uint64_t>((most * 8 + 127) / 128, 16ull * (uint32_t)ctx->sm_count);
+                ca.task_in = level & 1u ? tb : ta; ca.task_wide_in = level & 1u ? wb : wa;
+                ca.task_out = level & 1u ? ta : tb; ca.task_wide_out = level & 1u ? wa : wb;
+                k_collapse<<<grid, 128, 0, st>>>(ca, level);
+            }
+            cudaMemcpyAsync(&back, words, sizeof(back), cudaMemcpyDeviceToHost, st);
+            cudaMemcpyAsync(&bflag, flags + nint, 4, cudaMemcpyDeviceToHost, st);
+            cudaMemcpyAsync(&dflag, sah_flags + nd, 4, cudaMemcpyDeviceToHost, st);
             if ((s = cuda_check(ctx, cudaStreamSynchronize(st), "bvh: collapse"))) goto done;
-            ntask = cnt3[2];
-            // the nodes this level allocated are the next level
-            if (cnt3[0] > B.level_off.back()) B.level_off.push_back(cnt3[0]);
-            std::swap(ta, tb);
-            std::swap(wa, wb);
-            depth++;
-            if (depth > 200) { s = fail(ctx, XR_ERR_OVERFLOW, "bvh: collapse did not terminate"); goto done; }
+            if (ploc && back.made != n - 1) {
+                s = fail(ctx, XR_ERR_STATE, "bvh: clustering built the wrong number of nodes");
+                goto done;
+            }
+            if (back.counters[3] || bflag || dflag) { s = fail(ctx, XR_ERR_STATE, "bvh: inconsistent radix tree"); goto done; }
+            if (back.level_count[level] == 0u) break;
+            if (level + 8u > 200u) { s = fail(ctx, XR_ERR_OVERFLOW, "bvh: collapse did not terminate"); goto done; }
+            until = level + 8u;
         }
-        uint32_t ch[4], bflag = 0, dflag = 0;
-        cudaMemcpy(ch, counters, sizeof(ch), cudaMemcpyDeviceToHost);
-        cudaMemcpy(&bflag, flags + nint, 4, cudaMemcpyDeviceToHost);
-        if (sah) cudaMemcpy(&dflag, sah_flags + nint, 4, cudaMemcpyDeviceToHost);
-        bflag |= dflag;
-        if (ch[3] || bflag) { s = fail(ctx, XR_ERR_STATE, "bvh: inconsistent radix tree"); goto done; }
-        if (ch[1] != n) { s = fail(ctx, XR_ERR_STATE, "bvh: triangle slots do not match the primitive count"); goto done; }
+        if (back.counters[1] != n) { s = fail(ctx, XR_ERR_STATE, "bvh: triangle slots do not match the primitive count"); goto done; }
+        // the nodes each level allocated are the next level
+        B.level_off.push_back(0u);
+        uint32_t depth = 0;
+        for (; back.level_count[depth]; depth++) B.level_off.push_back(B.level_off.back() + back.level_count[depth]);
+        const uint32_t n_nodes = back.counters[0];
         if (B.nodes_into) B.nodes = B.nodes_into;
-        else if ((s = dalloc(ctx, &B.nodes, ch[0]))) goto done;
-        cudaMemcpyAsync(B.nodes, nodes_tmp, (size_t)ch[0] * sizeof(WideNode), cudaMemcpyDeviceToDevice, st);
+        else if ((s = dalloc(ctx, &B.nodes, n_nodes))) goto done;
+        cudaMemcpyAsync(B.nodes, nodes_tmp, (size_t)n_nodes * sizeof(WideNode), cudaMemcpyDeviceToDevice, st);
         cudaEventRecord(e1, st);
         if ((s = cuda_check(ctx, cudaStreamSynchronize(st), "bvh: finish"))) goto done;
-        B.n_nodes = ch[0];
-        B.n_slots = ch[1];
+        float amax;
+        memcpy(&amax, &back.bounds[6], 4);
+        B.emin = finest_exponent(amax, B.emin_floor);
+        B.n_nodes = n_nodes;
+        B.n_slots = n;
         B.depth = depth;
         cudaEventElapsedTime(&B.ms, e0, e1);
     }
 done:
-    sfree(ctx, tlo); sfree(ctx, thi); sfree(ctx, k0); sfree(ctx, k1); sfree(ctx, v0); sfree(ctx, v1); sfree(ctx, bounds);
-    sfree(ctx, hist); sfree(ctx, left); sfree(ctx, right); sfree(ctx, pint); sfree(ctx, pleaf); sfree(ctx, flags);
-    sfree(ctx, range); sfree(ctx, nlo); sfree(ctx, nhi); sfree(ctx, ta); sfree(ctx, tb); sfree(ctx, wa); sfree(ctx, wb);
-    sfree(ctx, counters); sfree(ctx, nodes_tmp);
-    sfree(ctx, sah_cost); sfree(ctx, sah_dec); sfree(ctx, sah_flags);
+    sfree(ctx, scratch);
     cudaEventDestroy(e0); cudaEventDestroy(e1);
     if (s != XR_OK) {
         if (!B.slots_into) cudaFree(B.slots);
