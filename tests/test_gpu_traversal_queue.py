@@ -57,3 +57,33 @@ def test_few_rays_and_crowded_nodes(n_rays, tris, size):
             ga, _, _ = r.trace(rays, any_hit=True)
             assert np.array_equal(ga >= 0, hit), (refill, batch)
         assert r.stats().error_flags == 0
+
+
+@pytest.mark.parametrize("n_rays", [1, 31, 33, 1000])
+@pytest.mark.parametrize("copies", [1, 7, 40])
+def test_few_rays_in_an_instanced_world(n_rays, copies):
+    """Overlapping instances of crowded soups: lanes that wait for their tests before they
+    leave an instance, and for others before they enter one; groups beyond the closest hit
+    are dropped."""
+    rng = np.random.default_rng(copies)
+    scenes = [_soup(200, 0.5, 1), _soup(9, 1.0, 2)]
+    inst = []
+    for i in range(copies):
+        m = np.zeros((3, 4), np.float32)
+        m[:, :3] = np.linalg.qr(rng.standard_normal((3, 3)))[0] * rng.uniform(0.4, 1.5)
+        m[:, 3] = rng.uniform(-1, 1, 3)
+        inst.append((i % 2, m))
+    world = ob.OracleWorld([ob.OracleScene.from_scene(s) for s in scenes])
+    world.set_instances(inst)
+    rays = _rays(n_rays, n_rays)
+    c = world.trace_instanced(rays)
+    with xr.Renderer(8, 8) as r:
+        r.upload_scenes(scenes)
+        r.set_instances(inst)
+        for refill, batch in ((0, 0), (1, 1), (32, 32)):
+            r.set_tuning(refill_min=refill, postpone_below=batch)
+            g = r.trace_instanced(rays)
+            for name, x, y in zip(("prim", "instance", "t", "bary"), g, c):
+                assert np.array_equal(np.asarray(x).view(np.uint32), np.asarray(y).view(np.uint32)), (name, refill, batch)
+            assert np.array_equal(r.trace_instanced(rays, any_hit=True)[0] >= 0, c[0] >= 0)
+        assert r.stats().error_flags == 0
