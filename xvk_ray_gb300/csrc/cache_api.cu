@@ -145,16 +145,20 @@ xr_status validate(const Context* c, const XrCacheParams* p) {
     return XR_OK;
 }
 
-// Uploads API samples and packs them into records (stride 2: query, 3: training).
+// Uploads API samples and packs them into records (stride 2: query, 3: training), in
+// stream order: the caller's array is read until the call's xr_sync.
 xr_status upload_samples(Context* c, const XrCacheSample* s, uint32_t n, uint32_t stride, uint4* rec) {
-    XrCacheSample* d = nullptr;
-    xr_status st = cuda_check(c, cudaMalloc((void**)&d, (size_t)n * sizeof(XrCacheSample)), "cache samples");
+    void* d = nullptr;
+    const size_t bytes = (size_t)n * sizeof(XrCacheSample);
+    xr_status st = stage_alloc(c, &d, bytes, "cache samples");
     if (st) return st;
-    st = cuda_check(c, cudaMemcpyAsync(d, s, (size_t)n * sizeof(XrCacheSample), cudaMemcpyHostToDevice, c->stream),
-                    "cache samples upload");
-    if (!st) launch_cache_pack(d, n, rec, stride, c->stream);
-    if (!st) st = cuda_check(c, cudaStreamSynchronize(c->stream), "cache pack");
-    cudaFree(d);
+    st = cuda_check(c, cudaMemcpyAsync(d, s, bytes, cudaMemcpyHostToDevice, c->stream), "cache samples upload");
+    if (!st) {
+        launch_cache_pack((const XrCacheSample*)d, n, rec, stride, c->stream);
+        st = cuda_check(c, cudaGetLastError(), "cache pack");
+    }
+    if (st) cudaStreamSynchronize(c->stream);
+    stage_free(c, d, bytes);
     return st;
 }
 
@@ -352,13 +356,17 @@ xr_status xr_cache_query(XrContext* c, const XrCacheSample* smp, uint32_t n, flo
     CacheState& cs = c->cache;
     if ((s = upload_samples(c, smp, n, 2u, cs.queries))) return s;
     float* d_out = nullptr;
-    if ((s = cuda_check(c, cudaMalloc((void**)&d_out, (size_t)n * 12), "cache query output"))) return s;
+    if ((s = stage_alloc(c, (void**)&d_out, (size_t)n * 12, "cache query output"))) {
+        cudaStreamSynchronize(c->stream);   // the samples' upload
+        return s;
+    }
     launch_cache_infer(cs, cs.queries, nullptr, n, d_out, nullptr, c->d_counters + kCntError, c->sm_count, c->stream);
     s = cuda_check(c, cudaGetLastError(), "cache query launch");
     if (!s) s = cuda_check(c, cudaMemcpyAsync(out_rgb, d_out, (size_t)n * 12, cudaMemcpyDeviceToHost, c->stream),
                            "cache query copy");
     if (!s) s = xr_sync(c);
-    cudaFree(d_out);
+    else cudaStreamSynchronize(c->stream);
+    stage_free(c, d_out, (size_t)n * 12);
     cs.frame_used = false;
     return s;
 }
@@ -381,6 +389,7 @@ xr_status xr_cache_train(XrContext* c, const XrCacheSample* smp, uint32_t n, int
     float l = 0.0f;
     if (!s) s = cuda_check(c, cudaMemcpyAsync(&l, cs.loss, 4, cudaMemcpyDeviceToHost, c->stream), "cache loss");
     if (!s) s = xr_sync(c);
+    else cudaStreamSynchronize(c->stream);
     cs.grads_dirty = apply == 0;
     cs.frame_used = false;
     if (loss) *loss = l;

@@ -48,6 +48,17 @@ void pool_free(Context* ctx, void* p) {
     if (p) cudaFreeAsync(p, ctx->stream);
 }
 
+xr_status stage_alloc(Context* ctx, void** p, size_t bytes, const char* what) {
+    if (bytes <= kStagePooled) return pool_alloc_bytes(ctx, p, bytes, what);
+    *p = nullptr;
+    return cuda_check(ctx, cudaMalloc(p, bytes), what);
+}
+
+void stage_free(Context* ctx, void* p, size_t bytes) {
+    if (bytes <= kStagePooled) pool_free(ctx, p);
+    else cudaFree(p);   // waits for the device
+}
+
 void invalidate_graphs(Context* c) {
     for (int i = 0; i < 2; i++) {
         if (c->graph[i]) cudaGraphExecDestroy(c->graph[i]);
@@ -266,10 +277,11 @@ xr_status upload_ubo(Context* c, const XrUniformBufferObject* ubo) {
 
 }  // namespace
 
+namespace {
+
+// The device error word as xr_sync read it: new bits make an error status.
 xr_status check_flags(Context* c) {
-    uint32_t flags = 0;
-    xr_status s = cuda_check(c, cudaMemcpy(&flags, c->d_counters + kCntError, 4, cudaMemcpyDeviceToHost), "read device flags");
-    if (s) return s;
+    const uint32_t flags = *c->h_flags;
     const uint32_t fresh = flags & ~c->error_flags;
     if (fresh) {
         c->error_flags |= flags;
@@ -282,8 +294,6 @@ xr_status check_flags(Context* c) {
     }
     return XR_OK;
 }
-
-namespace {
 
 xr_status validate_params(const Context* c, const XrParams* p) {
     if (!p) return fail(c, XR_ERR_INVALID_ARGUMENT, "params: null");
@@ -366,6 +376,8 @@ xr_status xr_create(const XrDeviceDesc* desc, XrContext** out) {
     if ((s = cuda_check(c, cudaMemset(c->d_work, 0, 2 * sizeof(unsigned long long)), "work counters"))) goto bad;
     if ((s = cuda_check(c, cudaMalloc((void**)&c->d_ubo, sizeof(XrUniformBufferObject)), "ubo"))) goto bad;
     if ((s = cuda_check(c, cudaMallocHost((void**)&c->h_ubo, 2 * sizeof(XrUniformBufferObject)), "ubo staging"))) goto bad;
+    if ((s = cuda_check(c, cudaMallocHost((void**)&c->h_flags, sizeof(uint32_t)), "error word"))) goto bad;
+    *c->h_flags = 0u;
     for (int i = 0; i < 8; i++)
         if ((s = cuda_check(c, cudaEventCreate(&c->ev[i]), "event"))) goto bad;
     for (int i = 0; i < 8; i++)
@@ -402,6 +414,7 @@ void xr_destroy(XrContext* c) {
     free_lights(c);
     free_instances(c);
     if (c->h_ubo) cudaFreeHost(c->h_ubo);
+    if (c->h_flags) cudaFreeHost(c->h_flags);
     for (int i = 0; i < 8; i++) if (c->ev[i]) cudaEventDestroy(c->ev[i]);
     for (int i = 0; i < 8; i++) if (c->user_ev[i]) cudaEventDestroy(c->user_ev[i]);
     for (int i = 0; i < 2; i++) if (c->refit_ev[i]) cudaEventDestroy(c->refit_ev[i]);
@@ -952,7 +965,10 @@ xr_status xr_render_reference_views(XrContext* c, const XrUniformBufferObject* u
 xr_status xr_sync(XrContext* c) {
     if (!c) return fail(nullptr, XR_ERR_INVALID_ARGUMENT, "sync: null context");
     DeviceGuard g(c->device);
-    xr_status s = cuda_check(c, cudaStreamSynchronize(c->stream), "sync");
+    // the error word follows the work in stream order: one wait for both
+    xr_status s = cuda_check(c, cudaMemcpyAsync(c->h_flags, c->d_counters + kCntError, 4, cudaMemcpyDeviceToHost,
+                                                c->stream), "read device flags");
+    if (!s) s = cuda_check(c, cudaStreamSynchronize(c->stream), "sync");
     if (s) return s;
     if (c->copy_stream && (s = cuda_check(c, cudaStreamSynchronize(c->copy_stream), "sync (image reads)"))) return s;
     return check_flags(c);
@@ -1172,23 +1188,27 @@ static xr_status trace_host(XrContext* c, const float* rays, uint32_t n, int32_t
     if (n == 0) return XR_OK;
     if (!rays || !prim || !t || !bary) return fail(c, XR_ERR_INVALID_ARGUMENT, "trace: null array");
     DeviceGuard g(c->device);
-    float* dr = nullptr; int32_t* dp = nullptr; int32_t* di = nullptr; float* dt = nullptr; float* db = nullptr;
-    xr_status s = XR_OK;
-    if ((s = cuda_check(c, cudaMalloc((void**)&dr, (size_t)n * 32), "trace alloc")) ||
-        (s = cuda_check(c, cudaMalloc((void**)&dp, (size_t)n * 4), "trace alloc")) ||
-        (inst && (s = cuda_check(c, cudaMalloc((void**)&di, (size_t)n * 4), "trace alloc"))) ||
-        (s = cuda_check(c, cudaMalloc((void**)&dt, (size_t)n * 4), "trace alloc")) ||
-        (s = cuda_check(c, cudaMalloc((void**)&db, (size_t)n * 8), "trace alloc")))
-        goto out;
-    cudaMemcpyAsync(dr, rays, (size_t)n * 32, cudaMemcpyHostToDevice, c->stream);
-    if ((s = trace_device(c, dr, n, any_hit, dp, di, dt, db))) goto out;
-    cudaMemcpyAsync(prim, dp, (size_t)n * 4, cudaMemcpyDeviceToHost, c->stream);
-    if (inst) cudaMemcpyAsync(inst, di, (size_t)n * 4, cudaMemcpyDeviceToHost, c->stream);
-    cudaMemcpyAsync(t, dt, (size_t)n * 4, cudaMemcpyDeviceToHost, c->stream);
-    cudaMemcpyAsync(bary, db, (size_t)n * 8, cudaMemcpyDeviceToHost, c->stream);
-    s = xr_sync(c);
-out:
-    cudaFree(dr); cudaFree(dp); cudaFree(di); cudaFree(dt); cudaFree(db);
+    // One staging block: rays, barycentrics, t, primitives, instances (each 4 n bytes or a
+    // multiple, the rays first, so every array keeps its alignment).  Five device allocations
+    // and frees a call and a second wait for the error word took half of a 1000-ray call.
+    const size_t N = n, bytes = N * (32 + 8 + 4 + 4 + (inst ? 4 : 0));
+    char* d = nullptr;
+    xr_status s = stage_alloc(c, (void**)&d, bytes, "trace alloc");
+    if (s) return s;
+    float *dr = (float*)d, *db = (float*)(d + 32 * N), *dt = (float*)(d + 40 * N);
+    int32_t *dp = (int32_t*)(d + 44 * N), *di = inst ? (int32_t*)(d + 48 * N) : nullptr;
+    s = cuda_check(c, cudaMemcpyAsync(dr, rays, N * 32, cudaMemcpyHostToDevice, c->stream), "trace upload");
+    if (!s) s = trace_device(c, dr, n, any_hit, dp, di, dt, db);
+    if (!s) {
+        cudaMemcpyAsync(prim, dp, N * 4, cudaMemcpyDeviceToHost, c->stream);
+        if (inst) cudaMemcpyAsync(inst, di, N * 4, cudaMemcpyDeviceToHost, c->stream);
+        cudaMemcpyAsync(t, dt, N * 4, cudaMemcpyDeviceToHost, c->stream);
+        cudaMemcpyAsync(bary, db, N * 8, cudaMemcpyDeviceToHost, c->stream);
+        s = xr_sync(c);
+    } else {
+        cudaStreamSynchronize(c->stream);   // the caller's arrays are free again on return
+    }
+    stage_free(c, d, bytes);
     return s;
 }
 

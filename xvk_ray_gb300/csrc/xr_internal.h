@@ -331,6 +331,7 @@ struct Context {
     unsigned long long* d_work = nullptr;   // node visits, triangle tests of the last ray query
     uint64_t query_rays = 0;
     uint32_t error_flags = 0;
+    uint32_t* h_flags = nullptr;            // page-locked copy of the device error word (xr_sync)
     cudaEvent_t ev[8] = {};          // 0..3 frame passes, 4 end of cache training, 5 unused, 6/7 cache inference
     // The cache's inference runs on infer_stream beside the training paths' bounces 2..
     // (forked at infer_fork_ev once bounce 1's queries exist, joined by the temporal pass
@@ -385,7 +386,11 @@ inline xr_status pool_alloc(Context* ctx, T** p, size_t count, const char* what)
     return pool_alloc_bytes(ctx, (void**)p, (count ? count : 1) * sizeof(T), what);
 }
 void pool_free(Context* ctx, void* p);
-xr_status check_flags(Context* c);   // reads the sticky device error word; new bits -> error status
+// Staging of one call's host arrays: from the pool, which keeps it for the next call, up to
+// kStagePooled bytes; larger blocks come from the device and go back to it with the call.
+constexpr size_t kStagePooled = 32u << 20;
+xr_status stage_alloc(Context* ctx, void** p, size_t bytes, const char* what);
+void stage_free(Context* ctx, void* p, size_t bytes);   // in stream order
 
 // Makes `dev` current for the scope of a C ABI call and restores the caller's device.
 struct DeviceGuard {
