@@ -143,7 +143,7 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt_mask = (1u << lane) - 1u;
     uint32_t q_head = 0, q_count = 0;   // the queue, a ring; these are the same in all lanes
-    uint32_t pending = 0;               // rays (their lanes) with a queued test
+    uint32_t pending = 0;               // INST: queued_rays(), kept for the pops of level markers
     bool drained = false;
     bool helping = false;                // lanes have been sent to help; the same in all lanes
     uint32_t ray_id = kInvalid;          // the lane's ray (kInvalid: none)
@@ -237,6 +237,13 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
         }
         if (e.y & 0xFFu) take_child(e);
     };
+    // Rays (their lanes) with a queued test.
+    auto queued_rays = [&]() {
+        uint32_t m = 0u;
+        for (uint32_t i = 0; i < q_count; i += 32u)
+            m |= __reduce_or_sync(FULL, i + lane < q_count ? 1u << sh.q_lane[(q_head + i + lane) & (kTriQueue - 1u)] : 0u);
+        return m;
+    };
     // One queued test per lane, the oldest first (all lanes of the warp call this).
     auto run_tests = [&]() {
         __syncwarp();
@@ -260,12 +267,14 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
         const int32_t r_inst = INST ? __shfl_sync(FULL, cur_inst, owner) : -1;
         q_head = (q_head + k) & (kTriQueue - 1u);
         q_count -= k;
-        // Merge: of the lanes whose hit beats a finder's record one writes it, until no
-        // lane's hit beats its record (several hits of one ray in one batch are rare).
-        // A record only ever improves, so the order of the tests does not matter; each
-        // round settles at least one lane, so at most 32 follow.
-        while (true) {
-            if (hit) {
+        // Merge: of the lanes with a hit one per ray writes it if it beats the ray's record,
+        // until none is left (several hits of one ray in one batch are rare).  A record only
+        // ever improves, so the order of the tests does not matter; each round settles at
+        // least one lane, so at most 32 follow.
+        while (__any_sync(FULL, hit)) {
+            if (hit) sh.winner[owner] = (uint8_t)lane;
+            __syncwarp();
+            if (hit && sh.winner[owner] == lane) {
                 const float ct = sh.t[owner];
                 const int32_t cp = sh.prim[owner];
                 bool tie_wins = prim < cp;
@@ -273,25 +282,19 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
                     const int32_t ci = sh.inst[owner];
                     tie_wins = r_inst < ci || (r_inst == ci && prim < cp);
                 }
-                hit = ANY ? cp < 0 : (cp < 0 ? tt <= ct : (tt < ct || (tt == ct && tie_wins)));
-            }
-            if (!__any_sync(FULL, hit)) break;
-            if (hit) sh.winner[owner] = (uint8_t)lane;
-            __syncwarp();
-            if (hit && sh.winner[owner] == lane) {
-                sh.t[owner] = tt;
-                sh.prim[owner] = prim;
-                sh.bary[owner] = make_float2(b1, b2);
-                if (INST) sh.inst[owner] = r_inst;
+                if (ANY ? cp < 0 : (cp < 0 ? tt <= ct : (tt < ct || (tt == ct && tie_wins)))) {
+                    sh.t[owner] = tt;
+                    sh.prim[owner] = prim;
+                    sh.bary[owner] = make_float2(b1, b2);
+                    if (INST) sh.inst[owner] = r_inst;
+                }
                 hit = false;
             }
             __syncwarp();
         }
         if (!ANY) h_t = sh.t[of];
         else if (sh.prim[of] >= 0) { cur = kInvalid; tg_mask = 0u; sp = sb = 0; }   // occluded: nothing left to visit
-        // rays that still have a test queued
-        const uint32_t left = lane < q_count ? 1u << sh.q_lane[(q_head + lane) & (kTriQueue - 1u)] : 0u;
-        pending = q_count ? __reduce_or_sync(FULL, left) : 0u;
+        if (INST) pending = queued_rays();
     };
 
     while (true) {
@@ -299,7 +302,7 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
         const uint32_t n_run = __popc(__ballot_sync(FULL, cur != kInvalid && !(INST && tg_mask)));
         if (n_run + refill_min <= 32u) {
             const bool empty = cur == kInvalid && sp == sb && !(INST && tg_mask);
-            uint32_t busy = pending;   // rays with a queued test or a helper at work
+            uint32_t busy = INST ? pending : queued_rays();   // rays with a queued test or a helper at work
             if (HELP && helping) {
                 busy |= __reduce_or_sync(FULL, !empty && of != lane ? 1u << of : 0u);
                 if (empty) of = lane;
@@ -540,7 +543,7 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
                     }
                 }
                 q_count += total;
-                pending |= HELP && helping ? __reduce_or_sync(FULL, n ? 1u << of : 0u) : p0 | p1;
+                if (INST) pending |= p0 | p1;
                 more = __any_sync(FULL, tg_mask != 0u && (!INST || in_blas));
             }
             // a whole batch, or what there is when too few lanes have nodes to visit
