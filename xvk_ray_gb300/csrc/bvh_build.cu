@@ -651,21 +651,13 @@ __global__ void __launch_bounds__(128) k_collapse(CollapseArgs a, uint32_t level
         node_grid(plo, phi, emin, p3, e);
         uint8_t ql[3] = {0, 0, 0}, qh[3] = {0, 0, 0};
         if (there) child_q(lo, hi, p3, e, emin, ql, qh);
-        // leaf triangle offsets in slot order
-        uint32_t off = 0u;
-        for (uint32_t t = 0; t < 8u; t++) {
-            const uint32_t o = __shfl_sync(gm, leaf ? (slot << 8) | cnt : 0xFF00u, g0 + t);
-            if ((o >> 8) < slot) off += o & 0xFFu;
-        }
-        uint32_t meta = 0u;
-        if (internal) meta = 0x20u | (24u + slot);                      // one bit, at 24 + slot
-        else if (leaf) meta = (((1u << cnt) - 1u) << 5) | off;          // cnt bits, at the triangle offset
+        // leaf triangles in slot order
+        const uint32_t children = (imask << 24) | __reduce_or_sync(gm, leaf ? ((1u << cnt) - 1u) << (3u * slot) : 0u);
+        const uint32_t off = __popc(children & ((1u << (3u * slot)) - 1u));   // used by leaves (slot < 8)
         // the node: every lane's bytes at its slot
         const uint32_t sh = 8u * (slot & 3u);
         const bool w0 = there && slot < 4u, w1 = there && slot >= 4u;
-        uint32_t m[2], q[12];
-        m[0] = __reduce_or_sync(gm, w0 ? meta << sh : 0u);
-        m[1] = __reduce_or_sync(gm, w1 ? meta << sh : 0u);
+        uint32_t q[12];
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             q[2 * k] = __reduce_or_sync(gm, w0 ? (uint32_t)ql[k] << sh : 0u);
@@ -674,11 +666,11 @@ __global__ void __launch_bounds__(128) k_collapse(CollapseArgs a, uint32_t level
             q[6 + 2 * k + 1] = __reduce_or_sync(gm, w1 ? (uint32_t)qh[k] << sh : 0u);
         }
         uint4* dst = reinterpret_cast<uint4*>(a.nodes + widx);
+        WideNode cells;
+        set_cells(cells, e);
         if (c == 0u)
-            dst[0] = make_uint4(__float_as_uint(p3[0]), __float_as_uint(p3[1]), __float_as_uint(p3[2]),
-                                (uint32_t)(e[0] + 127) | ((uint32_t)(e[1] + 127) << 8) | ((uint32_t)(e[2] + 127) << 16) |
-                                    (imask << 24));
-        else if (c == 1u) dst[1] = make_uint4(child_base, tri_base, m[0], m[1]);
+            dst[0] = make_uint4(__float_as_uint(p3[0]), __float_as_uint(p3[1]), __float_as_uint(p3[2]), cells.cell_xy);
+        else if (c == 1u) dst[1] = make_uint4(child_base, tri_base, children, cells.cell_z);
         else if (c == 2u) dst[2] = make_uint4(q[0], q[1], q[2], q[3]);
         else if (c == 3u) dst[3] = make_uint4(q[4], q[5], q[6], q[7]);
         else if (c == 4u) dst[4] = make_uint4(q[8], q[9], q[10], q[11]);
@@ -744,13 +736,13 @@ __global__ void k_refit_level(WideNode* __restrict__ nodes, uint32_t first, uint
     const uint32_t w = first + blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= first + n) return;
     WideNode nd = nodes[w];
-    const uint32_t imask = nd.exyz_imask >> 24;
+    const uint32_t imask = nd.children >> 24;
     float4 clo[8], chi[8];
     float4 plo = make_float4(INFINITY, INFINITY, INFINITY, 0), phi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0);
     uint32_t present = 0;
     for (int s = 0; s < 8; s++) {
-        const uint32_t meta = (nd.meta[s >> 2] >> (8 * (s & 3))) & 0xFFu;
-        if (meta == 0u) continue;
+        const uint32_t bits = (nd.children >> (3 * s)) & 7u;
+        if (!((imask >> s) & 1u) && (bits == 0u)) continue;
         present |= 1u << s;
         if (imask & (1u << s)) {
             const uint32_t c = nd.child_base + __popc(imask & ((1u << s) - 1u));
@@ -758,7 +750,7 @@ __global__ void k_refit_level(WideNode* __restrict__ nodes, uint32_t first, uint
             chi[s] = box_hi[c];
         } else {
             float4 lo = make_float4(INFINITY, INFINITY, INFINITY, 0), hi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0);
-            const uint32_t off = meta & 31u, cnt = __popc(meta >> 5);
+            const uint32_t off = __popc(nd.children & ((1u << (3 * s)) - 1u)), cnt = __popc(bits);
             for (uint32_t j = 0; j < cnt; j++)
                 for (int v = 0; v < 3; v++) {
                     const float4 q = tris[3u * ((size_t)nd.tri_base + off + j) + v];
@@ -783,7 +775,7 @@ __global__ void k_refit_level(WideNode* __restrict__ nodes, uint32_t first, uint
         for (int k = 0; k < 3; k++) { ql[k][s] = cql[k]; qh[k][s] = cqh[k]; }
     }
     nd.px = p3[0]; nd.py = p3[1]; nd.pz = p3[2];
-    nd.exyz_imask = (uint32_t)(e[0] + 127) | ((uint32_t)(e[1] + 127) << 8) | ((uint32_t)(e[2] + 127) << 16) | (imask << 24);
+    set_cells(nd, e);
     pack_q(ql, qh, nd.q);
     nodes[w] = nd;
 }

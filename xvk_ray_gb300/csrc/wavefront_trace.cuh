@@ -156,7 +156,7 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
     uint2 stack[kStackRing];
     uint32_t sp = 0, sb = 0;             // a ring: the bottom moves up when a helper takes it
     uint32_t cur = kInvalid;             // the node to visit next (kInvalid: none)
-    uint32_t tg_base = 0, tg_mask = 0;
+    uint32_t tg_base = 0, tg_mask = 0;   // triangles found: first slot, hit bits; INST: instances (of that top-level node)
     bool in_blas = !INST;    // INST: the lane's ray is in an instance's object space
     int32_t cur_inst = -1;   // that instance
     // INST: the world-space ray and its box-test state, kept for instance entries
@@ -407,6 +407,7 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
 
         // ---- visit a node ----
         uint2 found = make_uint2(0u, 0u);   // the internal children hit
+        uint32_t tg_valid = 0u;             // the child mask tg_mask's bits are of (triangles)
         if (cur != kInvalid && !(INST && tg_mask)) {
             const uint32_t node = cur;
             cur = kInvalid;
@@ -420,12 +421,12 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
                 const uint4 w0 = __ldg(np + 0), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3),
                             w4 = __ldg(np + 4);
                 // per axis: S = 32768 * 2^e / d and A = (p - o) / d - S (see qplane)
-                const float sx = __uint_as_float((w0.w & 0xFFu) << 23) * idx * 32768.0f;
-                const float sy = __uint_as_float(((w0.w >> 8) & 0xFFu) << 23) * idy * 32768.0f;
-                const float sz = __uint_as_float(((w0.w >> 16) & 0xFFu) << 23) * idz * 32768.0f;
-                const float ax = (__uint_as_float(w0.x) - o.x) * idx - sx;
-                const float ay = (__uint_as_float(w0.y) - o.y) * idy - sy;
-                const float az = (__uint_as_float(w0.z) - o.z) * idz - sz;
+                const float sx = __uint_as_float(w0.w & 0xFFFF0000u) * idx;
+                const float sy = __uint_as_float(w0.w << 16) * idy;
+                const float sz = __uint_as_float(w1.w) * idz;
+                const float ax = __fmaf_rn(__uint_as_float(w0.x) - o.x, idx, -sx);
+                const float ay = __fmaf_rn(__uint_as_float(w0.y) - o.y, idy, -sy);
+                const float az = __fmaf_rn(__uint_as_float(w0.z) - o.z, idz, -sz);
                 const float tlimit = h_t * (1.0f + 1e-6f) + 1e-30f;
                 // near and far quantised planes per axis, chosen once per node from the
                 // sign bits of the direction (a negative axis enters through the high plane)
@@ -436,11 +437,10 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
                 const uint32_t yf0 = ny ? w2.z : w4.x, yf1 = ny ? w2.w : w4.y;
                 const uint32_t zn0 = nz ? w4.z : w3.x, zn1 = nz ? w4.w : w3.y;
                 const uint32_t zf0 = nz ? w3.x : w4.z, zf1 = nz ? w3.y : w4.w;
-                uint32_t hm = 0;   // bits 0..23 triangles, 24..31 internal children by slot
+                uint32_t hm = 0;   // the hit slots' bits of the child mask
                 int32_t near1 = 0x7FFFFFFF, near2 = 0x7FFFFFFF;   // the two nearest hit boxes: entry t, slot in the low bits
 #pragma unroll
                 for (uint32_t i = 0; i < 8; i++) {
-                    const uint32_t meta = __byte_perm(i < 4 ? w1.z : w1.w, 0u, 0x4440u | (i & 3u));
                     const float txn = __fmaf_rn(qplane(i < 4 ? xn0 : xn1, i & 3u), sx, ax);
                     const float txf = __fmaf_rn(qplane(i < 4 ? xf0 : xf1, i & 3u), sx, ax);
                     const float tyn = __fmaf_rn(qplane(i < 4 ? yn0 : yn1, i & 3u), sy, ay);
@@ -450,28 +450,29 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
                     const float tn = fmaxf(max3f(txn, tyn, tzn), tmin_box);
                     const float tf = fminf(min3f(txf, tyf, tzf), tlimit);
                     const bool box_hit = tn <= __fmaf_rn(tf, 1.0f + 2e-6f, 1e-30f);
-                    if (box_hit) hm |= __funnelshift_l(0u, meta >> 5, meta);
+                    if (box_hit) hm |= (7u << (3u * i)) | (1u << (24u + i));
                     if (!NEAR) continue;
                     const int32_t key = box_hit ? (__float_as_int(tn) & ~7) | (int32_t)i : 0x7FFFFFFF;
                     near2 = min(near2, max(near1, key));
                     near1 = min(near1, key);
                 }
                 // internal hits from slot order to near-to-far order (bit k = slot k ^ flip)
+                hm &= w1.z;
                 uint32_t ih = hm >> 24;
                 if (flip & 1u) ih = ((ih & 0x55u) << 1) | ((ih >> 1) & 0x55u);
                 if (flip & 2u) ih = ((ih & 0x33u) << 2) | ((ih >> 2) & 0x33u);
                 if (flip & 4u) ih = ((ih & 0x0Fu) << 4) | ((ih >> 4) & 0x0Fu);
-                found = make_uint2(w1.x, ih | ((w0.w >> 24) << 8));
+                found = make_uint2(w1.x, ih | ((w1.z >> 16) & 0xFF00u));
                 if (NEAR && ih) {
                     // The nearest hit box, when it is an internal child, is visited next and the
                     // second nearest bounds the rest from below; else the first child in octant
                     // order, and the nearest box is the bound.
                     const uint32_t s1 = (uint32_t)near1 & 7u;
-                    const bool is_node = ((w0.w >> 24) >> s1) & 1u;
+                    const bool is_node = (w1.z >> (24u + s1)) & 1u;
                     found.y |= (uint32_t)max(is_node ? near2 : near1, 0) & 0xFFFF0000u;
                     if (is_node) {
                         found.y &= ~(1u << (s1 ^ flip));
-                        cur = w1.x + __popc((w0.w >> 24) & ((1u << s1) - 1u));
+                        cur = w1.x + __popc((w1.z >> 24) & ((1u << s1) - 1u));
                         if (found.y & 0xFFu) {
                             if (sp - sb < (uint32_t)kStackSize) stack[sp++ & (kStackRing - 1u)] = found;
                             else overflow();
@@ -481,7 +482,8 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
                 }
                 // children come after their parent, so every descent ends
                 if (ih && w1.x <= node) { overflow(); cur = kInvalid; found.y = 0u; }
-                tg_base = w1.y;
+                tg_base = INST && !in_blas ? node : w1.y;
+                tg_valid = w1.z;
                 tg_mask = hm & 0x00FFFFFFu;
             }
         }
@@ -493,13 +495,14 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
         // (the set-up is long: a lane waits until several want it or few can go on)
         const bool enter = INST && !in_blas && tg_mask != 0u;
         if (INST && (n_run < kMinRunning || __popc(__ballot_sync(FULL, enter)) >= (int)kEnterMin) && enter) {
-            const uint32_t bit = __ffs(tg_mask) - 1u;
+            const uint4 w1 = __ldg(reinterpret_cast<const uint4*>(sc.tlas_nodes + tg_base) + 1);
+            const uint32_t slot = w1.y + __popc(w1.z & (tg_mask - 1u) & ~tg_mask);
             tg_mask &= tg_mask - 1u;
-            if (tg_base + bit >= sc.n_inst_slots || sp + 3u > (uint32_t)kStackSize) {
+            if (slot >= sc.n_inst_slots || sp + 3u > (uint32_t)kStackSize) {
                 overflow();
                 tg_mask = 0u;
             } else {
-                const float4* ip = sc.inst_slots + 4u * (tg_base + bit);
+                const float4* ip = sc.inst_slots + 4u * slot;
                 const float4 m0 = __ldg(ip), m1 = __ldg(ip + 1), m2 = __ldg(ip + 2), m3 = __ldg(ip + 3);
                 // the rest of the top-level work (the next node as a group of one), then the level marker
                 if (cur != kInvalid) stack[sp++ & (kStackRing - 1u)] = make_uint2(cur, 1u << flip);
@@ -537,7 +540,7 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
     #pragma unroll
                 for (uint32_t i = 0; i < 3; i++) {
                     if (i < n) {
-                        sh.q_slot[(at + i) & (kTriQueue - 1u)] = tg_base + (__ffs(tg_mask) - 1u);
+                        sh.q_slot[(at + i) & (kTriQueue - 1u)] = tg_base + __popc(tg_valid & (tg_mask - 1u) & ~tg_mask);
                         sh.q_lane[(at + i) & (kTriQueue - 1u)] = (uint8_t)of;
                         tg_mask &= tg_mask - 1u;
                     }

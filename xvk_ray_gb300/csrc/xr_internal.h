@@ -66,21 +66,31 @@ constexpr uint32_t kCounterWords = 128;
 constexpr uint32_t kMaxBounces = 31;
 
 // 8-wide compressed BVH node, 80 B (five 16-byte words).
-//  w0: origin p.xyz, byte-packed {e.x, e.y, e.z (biased by 127), internal mask}
-//  w1: child_base, tri_base, meta[0..3], meta[4..7]
+//  w0: origin p.xyz, the upper halves of cell x and cell y
+//  w1: child_base, tri_base, child mask, cell z
 //  w2..w4: q_lo.x[8], q_lo.y[8], q_lo.z[8], q_hi.x[8], q_hi.y[8], q_hi.z[8]
-// meta byte = (bits << 5) | position: a hit child contributes bits << position
-// to one 32-bit mask.  Empty: 0.  Leaf of 1..3 triangles at tri_base + offset:
-// bits = 1, 3 or 7 (unary count), position = offset (0..23).  Internal child in
-// slot s: bits = 1, position = 24 + s; it is node child_base + popc(imask & ((1 << s) - 1)).
+// A cell is 32768 times the grid's (a power of two): what the box test multiplies by.
+// Child mask: bit 24 + s for an internal child in slot s, which is node
+// child_base + popc of the bits 24 .. 24 + s - 1; bits 3 s .. of a leaf of 1..3 triangles,
+// each at tri_base + popc of the bits below its own.  A hit child so adds its slot's four
+// bits, the same in every node (one instruction a child; a byte of position and count per
+// child, unpacked, shifted and added, took four).
 struct alignas(16) WideNode {
     float px, py, pz;
-    uint32_t exyz_imask;
+    uint32_t cell_xy;
     uint32_t child_base, tri_base;
-    uint32_t meta[2];
+    uint32_t children;
+    uint32_t cell_z;
     uint32_t q[12];
 };
 static_assert(sizeof(WideNode) == 80, "wide node is 80 B");
+// The sign and exponent bits of a cell of exponent e (2^(e + 15); infinite from 2^128 on,
+// which makes every plane of the axis NaN and culls nothing), and back.
+__host__ __device__ inline uint32_t cell_exponent(int e) { return (uint32_t)(e + 142 < 255 ? e + 142 : 255); }
+__host__ __device__ inline void set_cells(WideNode& n, const int e[3]) {
+    n.cell_xy = (cell_exponent(e[0]) << 23) | (cell_exponent(e[1]) << 7);
+    n.cell_z = cell_exponent(e[2]) << 23;
+}
 
 struct DeviceScene {
     const float4* tri;        // 3 float4 per BVH triangle slot: v0 {xyz, prim id}, v1, v2
