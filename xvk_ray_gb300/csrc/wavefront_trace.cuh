@@ -523,30 +523,31 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
         }
 
         // ---- queue the triangles found ----
+        auto put_test = [&](uint32_t at) {
+            sh.q_slot[at & (kTriQueue - 1u)] = tg_base + __popc(tg_valid & (tg_mask - 1u) & ~tg_mask);
+            sh.q_lane[at & (kTriQueue - 1u)] = (uint8_t)of;
+            tg_mask &= tg_mask - 1u;
+        };
         while (true) {
-            // up to three per lane where the ring has room (few nodes give a lane more), else one
             const uint32_t n_tri = (!INST || in_blas) ? __popc(tg_mask) : 0u;
-            const uint32_t three = n_tri < 3u ? n_tri : 3u;
-            const uint32_t p0 = __ballot_sync(FULL, three & 1u), p1 = __ballot_sync(FULL, three & 2u);
-            uint32_t total = __popc(p0) + 2u * __popc(p1);
+            const uint32_t m = __ballot_sync(FULL, n_tri != 0u);
             bool more = false;
-            if (total) {
-                uint32_t at = q_head + q_count + __popc(p0 & lt_mask) + 2u * __popc(p1 & lt_mask), n = three;
-                if (q_count + total > kTriQueue) {
-                    total = __popc(p0 | p1);
-                    at = q_head + q_count + __popc((p0 | p1) & lt_mask);
-                    n = three ? 1u : 0u;
+            if (m) {
+                const uint32_t tail = q_head + q_count;
+                if (q_count + 3u * __popc(m) <= kTriQueue) {
+                    // up to three per lane, where few lanes have any (few nodes give a lane more)
+                    const uint32_t n = n_tri < 3u ? n_tri : 3u;
+                    const uint32_t p0 = __ballot_sync(FULL, n & 1u), p1 = __ballot_sync(FULL, n & 2u);
+                    const uint32_t at = tail + __popc(p0 & lt_mask) + 2u * __popc(p1 & lt_mask);
+                    if (n > 0u) put_test(at);
+                    if (n > 1u) put_test(at + 1u);
+                    if (n > 2u) put_test(at + 2u);
+                    q_count += __popc(p0) + 2u * __popc(p1);
+                } else {
+                    if (n_tri) put_test(tail + __popc(m & lt_mask));
+                    q_count += __popc(m);
                 }
-    #pragma unroll
-                for (uint32_t i = 0; i < 3; i++) {
-                    if (i < n) {
-                        sh.q_slot[(at + i) & (kTriQueue - 1u)] = tg_base + __popc(tg_valid & (tg_mask - 1u) & ~tg_mask);
-                        sh.q_lane[(at + i) & (kTriQueue - 1u)] = (uint8_t)of;
-                        tg_mask &= tg_mask - 1u;
-                    }
-                }
-                q_count += total;
-                if (INST) pending |= p0 | p1;
+                if (INST) pending |= m;
                 more = __any_sync(FULL, tg_mask != 0u && (!INST || in_blas));
             }
             // a whole batch, or what there is when too few lanes have nodes to visit
