@@ -21,6 +21,7 @@
 // as the CPU oracle); only the order of the work differs, which the closest-hit
 // rule makes irrelevant for the result.
 #pragma once
+#include <type_traits>
 #include "traverse.cuh"
 
 namespace xr {
@@ -40,7 +41,12 @@ constexpr uint32_t kLevelBit = 0x40000000u;      // stack entry marks the return
 // before it leaves an instance, so the batch is smaller (dynamic world, 256 instances, three
 // renderers alternating: 6.42 ms a frame with 32, 6.29 with 24, 6.30 with 16).
 template <bool INST> constexpr uint32_t kTestBatch = INST ? 16u : 32u;
-constexpr uint32_t kRefillMin = XR_REFILL_MIN;     // default: finished lanes before a refill
+// Default: finished lanes before a refill.  Rays end soon in a small tree, so a refill (some
+// 200 instructions) serves more lanes there; in a large one idle lanes cost more.  Frames of
+// three contexts at 1600 x 1000, 8 and 20: 2.4k nodes 700 / 666 us, 4.8k 766 / 736, 9.7k
+// 883 / 858, 19k 958 / 954; 853 x 479 over 14k nodes 197 / 203, 1080p over 163k 1616 / 1659.
+constexpr uint32_t kRefillMin = XR_REFILL_MIN;
+constexpr uint32_t kRefillMinSmall = 20, kSmallTree = 12288;   // nodes
 constexpr uint32_t kMinRunning = XR_MIN_RUNNING;   // fewer lanes with nodes to visit: test what is queued
 constexpr uint32_t kEnterMin = XR_ENTER_MIN;       // lanes that want an instance before they enter together
 constexpr float kMinDir = 1e-20f;                 // smallest direction component seen by the box test
@@ -138,7 +144,7 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
     constexpr uint32_t FULL = 0xFFFFFFFFu;
     uint32_t n_visits = 0, n_tests = 0;
     // queue tuning of the context (0: the defaults)
-    const uint32_t refill_min = sc.refill_min ? sc.refill_min : kRefillMin;
+    const uint32_t refill_min = sc.refill_min ? sc.refill_min : !INST && sc.n_nodes < kSmallTree ? kRefillMinSmall : kRefillMin;
     const uint32_t batch = sc.postpone_below ? sc.postpone_below : kTestBatch<INST>;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt_mask = (1u << lane) - 1u;
@@ -186,13 +192,15 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
     };
     // A bound was exceeded: the ray goes on without what lies beyond it, the call fails.
     auto overflow = [&]() { atomicOr(err, (uint32_t)XR_DEVFLAG_STACK_OVERFLOW); };
+    // The stack is a ring once helpers take groups from its bottom, not before.
+    auto slot_of = [&](uint32_t i, auto tail) -> uint2& { return stack[decltype(tail)::value ? i & (kStackRing - 1u) : i]; };
     // Takes the first child of a group as the node to visit next; the rest goes on the stack.
-    auto take_child = [&](uint2 e) {
+    auto take_child = [&](uint2 e, auto tail) {
         const uint32_t k = __ffs(e.y) - 1u;
         e.y &= e.y - 1u;
         cur = e.x + __popc((e.y >> 8) & ((1u << (k ^ flip)) - 1u));
         if (e.y & 0xFFu) {
-            if (sp - sb < (uint32_t)kStackSize) stack[sp++ & (kStackRing - 1u)] = e;
+            if (sp - sb < (uint32_t)kStackSize) slot_of(sp++, tail) = e;
             else overflow();
         }
     };
@@ -212,10 +220,10 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
         }
     };
     // The next node: from the group `e` the last visit found, else from the stack.
-    auto next_node = [&](uint2 e) {
+    auto next_node = [&](uint2 e, auto tail) {
         if (cur != kInvalid || (INST && tg_mask && !in_blas)) return;
         while (!(e.y & 0xFFu) && sp != sb) {
-            e = stack[(sp - 1u) & (kStackRing - 1u)];
+            e = slot_of(sp - 1u, tail);
             if (INST && e.y == kLevelBit) {
                 if (tg_mask || ((pending >> lane) & 1u)) break;   // its tests still need this object space
                 // back to the top level: the world-space ray
@@ -235,7 +243,7 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
             }
             --sp;
         }
-        if (e.y & 0xFFu) take_child(e);
+        if (e.y & 0xFFu) take_child(e, tail);
     };
     // Rays (their lanes) with a queued test.
     auto queued_rays = [&]() {
@@ -245,7 +253,8 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
         return m;
     };
     // One queued test per lane, the oldest first (all lanes of the warp call this).
-    auto run_tests = [&]() {
+    auto run_tests = [&](auto tail) {
+        const uint32_t ray = decltype(tail)::value ? of : lane;
         __syncwarp();
         const uint32_t k = min(q_count, 32u);
         const uint32_t at = (q_head + lane) & (kTriQueue - 1u);
@@ -292,18 +301,22 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
             }
             __syncwarp();
         }
-        if (!ANY) h_t = sh.t[of];
-        else if (sh.prim[of] >= 0) { cur = kInvalid; tg_mask = 0u; sp = sb = 0; }   // occluded: nothing left to visit
+        if (!ANY) h_t = sh.t[ray];
+        else if (sh.prim[ray] >= 0) { cur = kInvalid; tg_mask = 0u; sp = sb = 0; }   // occluded: nothing left to visit
         if (INST) pending = queued_rays();
     };
 
-    while (true) {
+    // One round: finished rays out and new ones in, a node per lane, the tests it gave.
+    // `tail`: the ray queue is empty and lanes may help each other; what that takes stays
+    // out of the rounds before (6% of their instructions).  False once no ray is left.
+    auto round = [&](auto tail) -> bool {
+        constexpr bool TAIL = decltype(tail)::value;
         // lanes with a node to visit (not those that wait to enter an instance)
         const uint32_t n_run = __popc(__ballot_sync(FULL, cur != kInvalid && !(INST && tg_mask)));
         if (n_run + refill_min <= 32u) {
             const bool empty = cur == kInvalid && sp == sb && !(INST && tg_mask);
             uint32_t busy = INST ? pending : queued_rays();   // rays with a queued test or a helper at work
-            if (HELP && helping) {
+            if (TAIL && helping) {
                 busy |= __reduce_or_sync(FULL, !empty && of != lane ? 1u << of : 0u);
                 if (empty) of = lane;
             }
@@ -334,7 +347,7 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
                     }
                 }
                 const uint32_t idle = __ballot_sync(FULL, ray_id == kInvalid);
-                if (idle && !drained) {
+                if (!TAIL && idle && !drained) {
                     const uint32_t n_idle = __popc(idle);
                     uint32_t base = 0;
                     if (lane == 0) base = atomicAdd(next, n_idle);
@@ -368,9 +381,9 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
                         }
                     }
                 }
-                if (!__any_sync(FULL, ray_id != kInvalid)) break;
+                if (!__any_sync(FULL, ray_id != kInvalid)) return false;
             }
-            if (HELP && drained) {
+            if (TAIL) {
                 const bool idle = ray_id == kInvalid && of == lane;
                 const uint32_t m_idle = __ballot_sync(FULL, idle), m_give = __ballot_sync(FULL, sp != sb);
                 const uint32_t n = min(__popc(m_idle), __popc(m_give));
@@ -379,7 +392,7 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
                     const uint32_t r_give = __popc(m_give & lt_mask), r_take = __popc(m_idle & lt_mask);
                     uint2 e = make_uint2(0u, 0u);
                     if (sp != sb && r_give < n) {
-                        e = stack[sb++ & (kStackRing - 1u)];
+                        e = slot_of(sb++, tail);
                         sh.winner[r_give] = (uint8_t)lane;
                     }
                     __syncwarp();
@@ -399,7 +412,7 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
                     of = __shfl_sync(FULL, of, from);
                     if (take) {
                         sp = sb = 0u;
-                        take_child(e);
+                        take_child(e, tail);
                     }
                 }
             }
@@ -474,7 +487,7 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
                         found.y &= ~(1u << (s1 ^ flip));
                         cur = w1.x + __popc((w1.z >> 24) & ((1u << s1) - 1u));
                         if (found.y & 0xFFu) {
-                            if (sp - sb < (uint32_t)kStackSize) stack[sp++ & (kStackRing - 1u)] = found;
+                            if (sp - sb < (uint32_t)kStackSize) slot_of(sp++, tail) = found;
                             else overflow();
                         }
                         found.y = 0u;
@@ -488,8 +501,8 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
             }
         }
 
-        if (!INST || !tg_mask || in_blas) next_node(found);
-        else if (found.y & 0xFFu) take_child(found);   // top level: instances found go first
+        if (!INST || !tg_mask || in_blas) next_node(found, tail);
+        else if (found.y & 0xFFu) take_child(found, tail);   // top level: instances found go first
 
         // ---- instances found in a top-level node: enter one in object space ----
         // (the set-up is long: a lane waits until several want it or few can go on)
@@ -505,9 +518,9 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
                 const float4* ip = sc.inst_slots + 4u * slot;
                 const float4 m0 = __ldg(ip), m1 = __ldg(ip + 1), m2 = __ldg(ip + 2), m3 = __ldg(ip + 3);
                 // the rest of the top-level work (the next node as a group of one), then the level marker
-                if (cur != kInvalid) stack[sp++ & (kStackRing - 1u)] = make_uint2(cur, 1u << flip);
-                if (tg_mask) stack[sp++ & (kStackRing - 1u)] = make_uint2(tg_base, tg_mask | kTriGroupBit);
-                stack[sp++ & (kStackRing - 1u)] = make_uint2(0u, kLevelBit);
+                if (cur != kInvalid) slot_of(sp++, tail) = make_uint2(cur, 1u << flip);
+                if (tg_mask) slot_of(sp++, tail) = make_uint2(tg_base, tg_mask | kTriGroupBit);
+                slot_of(sp++, tail) = make_uint2(0u, kLevelBit);
                 tg_mask = 0u;
                 o = xform_point(m0, m1, m2, wo);
                 const float3 od = xform_dir(m0, m1, m2, wd);
@@ -525,7 +538,7 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
         // ---- queue the triangles found ----
         auto put_test = [&](uint32_t at) {
             sh.q_slot[at & (kTriQueue - 1u)] = tg_base + __popc(tg_valid & (tg_mask - 1u) & ~tg_mask);
-            sh.q_lane[at & (kTriQueue - 1u)] = (uint8_t)of;
+            sh.q_lane[at & (kTriQueue - 1u)] = (uint8_t)(TAIL ? of : lane);
             tg_mask &= tg_mask - 1u;
         };
         while (true) {
@@ -551,10 +564,15 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
                 more = __any_sync(FULL, tg_mask != 0u && (!INST || in_blas));
             }
             // a whole batch, or what there is when too few lanes have nodes to visit
-            while (q_count >= batch || (!more && q_count && n_run < kMinRunning)) run_tests();
+            while (q_count >= batch || (!more && q_count && n_run < kMinRunning)) run_tests(tail);
             if (!more) break;
         }
-    }
+        return true;
+    };
+    bool going = true;
+    while (going && !(HELP && drained)) going = round(std::false_type{});
+    if (HELP)
+        while (going) going = round(std::true_type{});
     if (work) {
         atomicAdd(&work[0], (unsigned long long)n_visits);
         atomicAdd(&work[1], (unsigned long long)n_tests);
