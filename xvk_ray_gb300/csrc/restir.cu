@@ -740,6 +740,14 @@ __device__ __forceinline__ void load_wide(const FrameArgs& fa, float4* const* pl
     r.ns = xyz(c); r.m = __float_as_uint(c.w);
     r.f = xyz(d); r.code = 0u;
 }
+// Without f: the merges of the spatial pass do not look at it.
+__device__ __forceinline__ void load_wide_no_f(float4* const* planes, uint32_t i, Res& r) {
+    float4 a = planes[0][i], b = planes[1][i], c = planes[2][i];
+    r.xs = xyz(a); r.W = a.w;
+    r.L = xyz(b); r.w_sum = b.w;
+    r.ns = xyz(c); r.m = __float_as_uint(c.w);
+    r.f = f3(0.0f, 0.0f, 0.0f); r.code = 0u;
+}
 __device__ __forceinline__ void store_wide(float4* const* planes, uint32_t i, const Res& r) {
     planes[0][i] = f4(r.xs, r.W);
     planes[1][i] = f4(r.L, r.w_sum);
@@ -783,7 +791,11 @@ __device__ __forceinline__ float3 mat_albedo_over_pi(const FrameArgs& fa, uint32
 }
 
 // ---- temporal, compat layout (the reference's fields and quirks) ----
-__global__ void __launch_bounds__(256) k_temporal_compat(FrameArgs fa, const XrUniformBufferObject* __restrict__ u, bool out_here) {
+// The compat passes wait for their gathers (a third of the issue slots used at 24 warps an
+// SM): 9 blocks of 128 an SM in 56 registers for temporal, 89 -> 78 us at 1920 x 1080 (5.9
+// TB/s), and 7 in 72 for spatial, which spills below that (7 / 8 / 9: 162 / 169 / 178 us).
+constexpr int kCompatBlock = 128;
+__global__ void __launch_bounds__(kCompatBlock, 9) k_temporal_compat(FrameArgs fa, const XrUniformBufferObject* __restrict__ u, bool out_here) {
     uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= fa.N) return;
     const PixView pv = pix_view(fa, p);
@@ -885,7 +897,9 @@ __device__ __forceinline__ float jacobian_of(float3 x_nb_view, float3 x_view, fl
 }
 
 // ---- spatial, compat layout ----
-__global__ void __launch_bounds__(256) k_spatial_compat(FrameArgs fa, const XrUniformBufferObject* __restrict__ u) {
+// Issue-bound once its gathers overlap (61% of the slots): the next neighbour's G-buffer words
+// are fetched with this one's reservoir, and f only for the sample kept: 197 -> 162 us.
+__global__ void __launch_bounds__(kCompatBlock, 7) k_spatial_compat(FrameArgs fa, const XrUniformBufferObject* __restrict__ u) {
     uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= fa.N) return;
     const PixView pv = pix_view(fa, p);
@@ -900,23 +914,35 @@ __global__ void __launch_bounds__(256) k_spatial_compat(FrameArgs fa, const XrUn
     if (length(xyz(nv)) == 0.0f) { write_out(fa, p, f3(0, 0, 0), false); return; }
     if (length(xyz(ns)) == 0.0f) { write_out(fa, p, f3(1, 1, 1), false); return; }
     const uint32_t mat = __float_as_uint(xv.w);
-    Res center; load_wide(fa, fa.rw, read_off + p, center);
+    Res center; load_wide_no_f(fa.rw, read_off + p, center);
     Res r; res_init(r);
-    res_merge(r, center, length(center.L), rng);
+    uint32_t win = kInvalid;   // the pixel whose sample is held: its f is gathered once, at the end
+    if (res_merge(r, center, length(center.L), rng)) win = p;
+    uint32_t nbi = pv.base + neighbor_index(x, y, pv.W, pv.H, 5.0f, rng);
+    float4 nxv = fa.s_xv[nbi], nnv = fa.s_nv[nbi];
     for (int i = 0; i < 6; i++) {
-        uint32_t nbi = pv.base + neighbor_index(x, y, pv.W, pv.H, 5.0f, rng);
-        float4 nxv = fa.s_xv[nbi], nnv = fa.s_nv[nbi];
-        if (length(xyz(nnv)) == 0.0f) continue;
-        float3 dd = xyz(xv) - xyz(nxv);
-        if (dot(dd, dd) > 0.1f) continue;
-        if (dot(xyz(nv), xyz(nnv)) < 0.8f) continue;
-        if (mat != __float_as_uint(nxv.w)) continue;
-        Res rn; load_wide(fa, fa.rw, read_off + nbi, rn);
-        float jac = jacobian_of(xyz(nxv), xyz(xv), rn.xs, rn.ns);
+        const float3 dd = xyz(xv) - xyz(nxv);
+        const bool similar = length(xyz(nnv)) != 0.0f && !(dot(dd, dd) > 0.1f) && !(dot(xyz(nv), xyz(nnv)) < 0.8f) &&
+                             mat == __float_as_uint(nxv.w);
+        const uint32_t at = nbi;
+        const float3 x_nb = xyz(nxv);
+        Res rn;
+        if (similar) load_wide_no_f(fa.rw, read_off + at, rn);
+        // a merge draws once: the next pick is known, and its words are on their way with this one's reservoir
+        uint32_t rng_merge = rng;
+        if (similar) (void)random_float(rng);
+        if (i < 5) {
+            nbi = pv.base + neighbor_index(x, y, pv.W, pv.H, 5.0f, rng);
+            nxv = fa.s_xv[nbi];
+            nnv = fa.s_nv[nbi];
+        }
+        if (!similar) continue;
+        float jac = jacobian_of(x_nb, xyz(xv), rn.xs, rn.ns);
         float ph = length(rn.L) * jac;
-        res_merge(r, rn, ph, rng);
+        if (res_merge(r, rn, ph, rng_merge)) win = at;
         if (ph == 0.0f) r.m -= rn.m;
     }
+    if (win != kInvalid) r.f = xyz(fa.rw[3][read_off + win]);
     r.m = min(r.m, 300u);
     float phf = length(r.L);
     r.W = (phf > 1e-6f && r.m > 0u) ? r.w_sum / ((float)r.m * phf) : 0.0f;
@@ -1535,8 +1561,7 @@ void launch_initial(const FrameArgs& fa, uint32_t nb, cudaStream_t st, void (*af
 }
 
 void launch_temporal(const FrameArgs& fa, bool write_image, cudaStream_t st) {
-    uint32_t blocks = (fa.N + 255u) / 256u;
-    if (fa.compat) k_temporal_compat<<<blocks, 256, 0, st>>>(fa, fa.ubo, write_image);
+    if (fa.compat) k_temporal_compat<<<(fa.N + kCompatBlock - 1u) / kCompatBlock, kCompatBlock, 0, st>>>(fa, fa.ubo, write_image);
     else {
         const uint32_t tb = fa.blk_temporal ? fa.blk_temporal : (uint32_t)XR_TEMPORAL_BLOCK;
         k_temporal<<<(fa.N + tb - 1u) / tb, tb, 0, st>>>(fa, fa.ubo, write_image);
@@ -1572,9 +1597,8 @@ void launch_accumulate_sample(const FrameArgs& fa, double* acc, cudaStream_t st)
 }
 
 void launch_spatial(const FrameArgs& fa, cudaStream_t st) {
-    uint32_t blocks = (fa.N + 255u) / 256u;
     if (fa.compat) {
-        k_spatial_compat<<<blocks, 256, 0, st>>>(fa, fa.ubo);
+        k_spatial_compat<<<(fa.N + kCompatBlock - 1u) / kCompatBlock, kCompatBlock, 0, st>>>(fa, fa.ubo);
         return;
     }
     const uint32_t sb = fa.blk_spatial ? fa.blk_spatial : (uint32_t)XR_SPATIAL_BLOCK;
