@@ -54,11 +54,20 @@ __device__ __forceinline__ void store_row(uint8_t* base, uint32_t r, const float
     }
 }
 
-// Row r of a K-major [*][64] bf16 operand -> 64 float values.
-__device__ __forceinline__ void load_row64(const uint8_t* base, uint32_t r, float* v) {
+// N columns from c0 of row r of a K-major [*][64] bf16 operand, written and read.
+template <int N>
+__device__ __forceinline__ void store_cols(uint8_t* base, uint32_t r, uint32_t c0, const float* v) {
 #pragma unroll
-    for (int c = 0; c < 64; c += 8) {
-        const uint4 w = *reinterpret_cast<const uint4*>(base + umma::kmajor_offset(r, c, 64));
+    for (int c = 0; c < N; c += 8)
+        *reinterpret_cast<uint4*>(base + umma::kmajor_offset(r, c0 + c, 64)) =
+            make_uint4(pack2(v[c], v[c + 1]), pack2(v[c + 2], v[c + 3]), pack2(v[c + 4], v[c + 5]),
+                       pack2(v[c + 6], v[c + 7]));
+}
+template <int N>
+__device__ __forceinline__ void load_cols(const uint8_t* base, uint32_t r, uint32_t c0, float* v) {
+#pragma unroll
+    for (int c = 0; c < N; c += 8) {
+        const uint4 w = *reinterpret_cast<const uint4*>(base + umma::kmajor_offset(r, c0 + c, 64));
         const uint32_t u[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -79,10 +88,10 @@ __host__ __device__ __forceinline__ uint32_t t_offset(uint32_t r, uint32_t k) {
     return (r >> 3) * kTSbo + (k >> 3) * kTLbo + (r & 7u) * 16u + (k & 7u) * 2u;
 }
 template <int ROWS>
-__device__ __forceinline__ void store_col_t(uint8_t* base, uint32_t col, const float* v) {
+__device__ __forceinline__ void store_col_t(uint8_t* base, uint32_t row0, uint32_t col, const float* v) {
 #pragma unroll
     for (int r = 0; r < ROWS; ++r)
-        *reinterpret_cast<uint16_t*>(base + t_offset((uint32_t)r, col)) = umma::bf16_bits(v[r]);
+        *reinterpret_cast<uint16_t*>(base + t_offset(row0 + (uint32_t)r, col)) = umma::bf16_bits(v[r]);
 }
 
 __device__ __forceinline__ void copy_image(uint8_t* dst, const uint8_t* __restrict__ src, uint32_t bytes) {
@@ -99,28 +108,26 @@ __device__ __forceinline__ void publish() {
     umma::fence_after_sync();
 }
 
-// D (+)= A[128][K] * B[N][K]^T, `steps` K = 16 steps; issued by one thread.
-__device__ __forceinline__ void gemm(uint32_t d_tmem, const uint8_t* A, const uint8_t* B, uint32_t K, uint32_t N,
-                                     uint32_t steps, bool accumulate) {
-    const uint32_t id = umma::idesc_bf16_f32(128, N);
-    const uint32_t a0 = umma::smem_u32(A), b0 = umma::smem_u32(B);
-    for (uint32_t s = 0; s < steps; ++s) {
-        const uint64_t ad = umma::smem_desc(a0 + 256u * s, 128u, K * 16u);
-        const uint64_t bd = umma::smem_desc(b0 + 256u * s, 128u, K * 16u);
-        umma::mma_bf16(d_tmem, ad, bd, id, (accumulate || s > 0) ? 1u : 0u);
-    }
+// D (+)= A[128][K] * B[N][K]^T in K / 16 steps; issued by one thread.  The steps' descriptors
+// differ in the address alone, 256 bytes or 16 units on.
+template <int K, uint32_t N>
+__device__ __forceinline__ void gemm(uint32_t d_tmem, const uint8_t* A, const uint8_t* B) {
+    constexpr uint32_t id = umma::idesc_bf16_f32(128, N);
+    const uint64_t ad = umma::smem_desc(umma::smem_u32(A), 128u, K * 16u);
+    const uint64_t bd = umma::smem_desc(umma::smem_u32(B), 128u, K * 16u);
+#pragma unroll
+    for (int s = 0; s < K / 16; ++s) umma::mma_bf16(d_tmem, ad + 16u * s, bd + 16u * s, id, s > 0 ? 1u : 0u);
 }
 
-// D (+)= A[128][128] * B[N][128]^T over the transposed (padded) layout; one thread.
-__device__ __forceinline__ void gemm_t(uint32_t d_tmem, const uint8_t* A, const uint8_t* B, uint32_t N,
-                                       bool accumulate) {
-    const uint32_t id = umma::idesc_bf16_f32(128, N);
-    const uint32_t a0 = umma::smem_u32(A), b0 = umma::smem_u32(B);
-    for (uint32_t s = 0; s < 8u; ++s) {   // K = 16 per step: two core matrices
-        const uint64_t ad = umma::smem_desc(a0 + 2u * kTLbo * s, kTLbo, kTSbo);
-        const uint64_t bd = umma::smem_desc(b0 + 2u * kTLbo * s, kTLbo, kTSbo);
-        umma::mma_bf16(d_tmem, ad, bd, id, (accumulate || s > 0) ? 1u : 0u);
-    }
+// D (+)= A[128][128] * B[64][128]^T over the transposed (padded) layout, two core matrices or
+// 2 kTLbo bytes a step; one thread.
+__device__ __forceinline__ void gemm_t(uint32_t d_tmem, const uint8_t* A, const uint8_t* B, bool accumulate) {
+    constexpr uint32_t id = umma::idesc_bf16_f32(128, 64);
+    const uint64_t ad = umma::smem_desc(umma::smem_u32(A), kTLbo, kTSbo);
+    const uint64_t bd = umma::smem_desc(umma::smem_u32(B), kTLbo, kTSbo);
+#pragma unroll
+    for (int s = 0; s < 8; ++s)
+        umma::mma_bf16(d_tmem, ad + 2u * kTLbo / 16u * s, bd + 2u * kTLbo / 16u * s, id, accumulate || s > 0 ? 1u : 0u);
 }
 
 // Every thread waits for the last commit; the outcome is the same in all threads.
@@ -132,21 +139,12 @@ __device__ __forceinline__ bool wait_mma(uint64_t* bar, uint32_t& phase) {
     return ok;
 }
 
-// 64 accumulator columns [c0, c0 + 64) of this thread's lane.
-__device__ __forceinline__ void tmem_row64(uint32_t taddr, float* v) {
-    umma::tmem_ld16(taddr, v);
-    umma::tmem_ld16(taddr + 16u, v + 16);
-    umma::tmem_ld16(taddr + 32u, v + 32);
-    umma::tmem_ld16(taddr + 48u, v + 48);
+// N accumulator columns (a multiple of 16) of this thread's lane.
+template <int N>
+__device__ __forceinline__ void tmem_cols(uint32_t taddr, float* v) {
+#pragma unroll
+    for (int c = 0; c < N; c += 16) umma::tmem_ld16(taddr + c, v + c);
     umma::tmem_wait_ld();
-}
-
-__device__ __forceinline__ void inputs_of(const Bounds& bnd, const __half2* table, const uint4* rec, uint32_t stride,
-                                          uint32_t i, float4& ra, uint4& rb, float* v) {
-    const uint4 a = rec[(size_t)i * stride], b = rec[(size_t)i * stride + 1];
-    ra = make_float4(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z), __uint_as_float(a.w));
-    rb = b;
-    network_inputs(bnd, table, ra, rb, v);
 }
 
 }  // namespace
@@ -155,17 +153,68 @@ __device__ __forceinline__ void inputs_of(const Bounds& bnd, const __half2* tabl
 // inference: MODE 0 writes out3[i] (test/API path), MODE 1 adds the prediction
 // (clamped at 0) to the candidate radiance cand_b[pixel].rgb of the frame.
 // ---------------------------------------------------------------------------
+// kInferGroups threads share a sample: the encoding's levels, the columns of a layer's
+// activations and the rest of the inputs are split between them.  The kernel waits for the
+// table's gathers (L1 hits half of them) and, layer by layer, for its own block: it wants warps
+// and L1.  Two threads a sample and three blocks an SM (24 warps, 156 of 256 KB shared) take
+// 99 us for the 1.3M queries of a 1080p frame and 40 for 65536; one thread and four blocks
+// (213 KB shared, a second wave) 153 and 77, two and four 161 and 80, two and two 116 and 38,
+// four and two 116 and 41, two and three with the largest carve-out 159 and 75.
+#ifndef XR_INFER_GROUPS
+#define XR_INFER_GROUPS 2
+#endif
+#ifndef XR_INFER_BLOCKS
+#define XR_INFER_BLOCKS 3
+#endif
+constexpr int kInferGroups = XR_INFER_GROUPS, kInferBlocks = XR_INFER_BLOCKS;
+
+// Features [C0, C1) of 64 of row r (multiples of 8).
+template <int C0, int C1>
+__device__ __forceinline__ void store_inputs(const Bounds& bnd, const __half2* __restrict__ table, float4 ra, uint4 rb,
+                                             bool valid, uint8_t* sX, uint32_t r) {
+    float v[8];
+    constexpr int kFeat = 2 * kLevels;
+    const float3 p = unit_pos(bnd, xyz(ra));
+#pragma unroll
+    for (int c = C0; c < C1; c += 8) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = 0.0f;
+        if (valid && c < kFeat) {
+#pragma unroll
+            for (int l = 0; l < 4; ++l) level_features(c / 2 + l, p, table, &v[2 * l]);
+        } else if (valid && c < kFeat + 16) {
+            float x[16];
+            other_inputs(rb, x);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = x[c - kFeat + j];
+        }
+        *reinterpret_cast<uint4*>(sX + umma::kmajor_offset(r, (uint32_t)c, kIn)) =
+            make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
+    }
+}
+// The inputs of group g of GROUPS of a sample.
+template <int GROUPS, int G = 0>
+__device__ __forceinline__ void store_group_inputs(uint32_t g, const Bounds& bnd, const __half2* __restrict__ table, float4 ra,
+                                                   uint4 rb, bool valid, uint8_t* sX, uint32_t r) {
+    constexpr int kF = 2 * kLevels / GROUPS;
+    if (g == (uint32_t)G) {
+        store_inputs<G * kF, (G + 1) * kF>(bnd, table, ra, rb, valid, sX, r);
+        store_inputs<2 * kLevels + G * kF, 2 * kLevels + (G + 1) * kF>(bnd, table, ra, rb, valid, sX, r);
+    }
+    if constexpr (G + 1 < GROUPS) store_group_inputs<GROUPS, G + 1>(g, bnd, table, ra, rb, valid, sX, r);
+}
+
 template <int MODE>
-__global__ void __launch_bounds__(128) k_cache_infer(const uint4* __restrict__ rec, const uint32_t* count_ptr,
-                                                     uint32_t count_host, Bounds bnd, const __half2* __restrict__ table,
-                                                     const uint8_t* __restrict__ w_fwd, float* __restrict__ out3,
-                                                     float4* __restrict__ cand_b, uint32_t* err) {
+__global__ void __launch_bounds__(kTile* kInferGroups, kInferBlocks)
+    k_cache_infer(const uint4* __restrict__ rec, const uint32_t* count_ptr, uint32_t count_host, Bounds bnd,
+                  const __half2* __restrict__ table, const uint8_t* __restrict__ w_fwd, float* __restrict__ out3,
+                  float4* __restrict__ cand_b, uint32_t* err) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sW = smem;                  // forward weight image
     uint8_t* sX = smem + kImageBytes;    // activations of the current layer
     __shared__ uint64_t bar;
     __shared__ uint32_t tslot;
-    const uint32_t tid = threadIdx.x, warp = tid >> 5;
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, row = tid % kTile, g = tid / kTile;
     const uint32_t count = count_ptr ? *(volatile const uint32_t*)count_ptr : count_host;
     const uint32_t ntiles = (count + kTile - 1u) / kTile;
     if (blockIdx.x >= ntiles) return;
@@ -177,36 +226,44 @@ __global__ void __launch_bounds__(128) k_cache_infer(const uint4* __restrict__ r
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = tslot;
-    const uint32_t lane_addr = tmem + ((warp * 32u) << 16);
+    const uint32_t lane_addr = tmem + (((warp & 3u) * 32u) << 16);
     uint32_t phase = 0;
     bool ok = true;
 
     for (uint32_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-        const uint32_t i = tile * kTile + tid;
+        const uint32_t i = tile * kTile + row;
         const bool valid = i < count;
-        float v[kIn];
-        float4 ra = make_float4(0, 0, 0, 0);
-        uint4 rb = make_uint4(0, 0, 0, 0);
-        if (valid) inputs_of(bnd, table, rec, 2u, i, ra, rb, v);
-        else {
-#pragma unroll
-            for (int j = 0; j < kIn; ++j) v[j] = 0.0f;
+        uint32_t pixel = 0u;
+        {
+            float4 ra = make_float4(0, 0, 0, 0);
+            uint4 rb = make_uint4(0, 0, 0, 0);
+            if (valid) {
+                const uint4 a = rec[(size_t)i * 2u];
+                rb = rec[(size_t)i * 2u + 1u];
+                ra = make_float4(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z), 0.0f);
+                pixel = a.w;
+            }
+            store_group_inputs<kInferGroups>(g, bnd, table, ra, rb, valid, sX, row);
         }
-        store_row<kIn>(sX, tid, v);
         for (int l = 0; l <= kHidden && ok; ++l) {
             publish();
             if (tid == 0) {
-                gemm(tmem, sX, sW + l * kLayerBytes, 64u, l < kHidden ? 64u : 16u, 4u, false);
+                if (l < kHidden) gemm<64, 64>(tmem, sX, sW + l * kLayerBytes);
+                else gemm<64, 16>(tmem, sX, sW + l * kLayerBytes);
                 umma::commit(&bar);
             }
             ok = wait_mma(&bar, phase);
             if (!ok) break;
             if (l < kHidden) {
-                tmem_row64(lane_addr, v);
+                // this group's columns of the row
+                constexpr int kN = kWidth / kInferGroups;
+                float v[kN];
+                tmem_cols<kN>(lane_addr + g * kN, v);
 #pragma unroll
-                for (int j = 0; j < kWidth; ++j) v[j] = fmaxf(v[j], 0.0f);
-                store_row<kIn>(sX, tid, v);
-            } else {
+                for (int j = 0; j < kN; ++j) v[j] = fmaxf(v[j], 0.0f);
+                store_cols<kN>(sX, row, g * kN, v);
+            } else if (g == 0u) {
+                float v[16];
                 umma::tmem_ld16(lane_addr, v);
                 umma::tmem_wait_ld();
                 if (valid) {
@@ -215,7 +272,6 @@ __global__ void __launch_bounds__(128) k_cache_infer(const uint4* __restrict__ r
                         out3[(size_t)i * 3 + 1] = v[1];
                         out3[(size_t)i * 3 + 2] = v[2];
                     } else {
-                        const uint32_t pixel = __float_as_uint(ra.w);
                         float3 L = f3(fmaxf(v[0], 0.0f), fmaxf(v[1], 0.0f), fmaxf(v[2], 0.0f));
                         if (!isfinite(L.x + L.y + L.z)) L = f3(0.0f, 0.0f, 0.0f);
                         float4 c = cand_b[pixel];
@@ -247,20 +303,29 @@ __device__ __forceinline__ uint32_t train_samples(const uint32_t* count_ptr, uin
 }
 
 // Sample j of the tiles is record perm[j] (the spatial order below); its unit
-// position goes to upos[j] for k_cache_scatter.
+// position goes to upos[j] for k_cache_scatter.  kEncodeGroups threads share a sample, a warp
+// one group's levels: one thread a sample left 13 warps an SM waiting for the table
+// (65536 samples 23.4 -> 19.9 us; four 20.8).
+#ifndef XR_ENCODE_GROUPS
+#define XR_ENCODE_GROUPS 2
+#endif
+constexpr uint32_t kEncodeGroups = XR_ENCODE_GROUPS;
 __global__ void __launch_bounds__(256) k_cache_encode(const uint4* __restrict__ rec, const uint32_t* __restrict__ perm,
                                                       const uint32_t* count_ptr, uint32_t count_host, uint32_t cap,
                                                       Bounds bnd, const __half2* __restrict__ table,
                                                       uint8_t* __restrict__ tiles, float4* __restrict__ upos) {
     const uint32_t n = train_samples(count_ptr, count_host, cap);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float v[kIn];
-        float4 ra;
-        uint4 rb;
-        inputs_of(bnd, table, rec, 3u, perm[i], ra, rb, v);
-        const float3 p = unit_pos(bnd, xyz(ra));
-        upos[i] = make_float4(p.x, p.y, p.z, 0.0f);
-        store_row<kIn>(tiles + (size_t)(i / kTile) * kActBytes, i % kTile, v);
+    for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < n * kEncodeGroups; u += gridDim.x * blockDim.x) {
+        const uint32_t row = u % kTile, g = u / kTile % kEncodeGroups, tile = u / (kTile * kEncodeGroups);
+        const uint32_t i = tile * kTile + row;
+        const uint4* q = rec + (size_t)perm[i] * 3u;
+        const uint4 a = q[0], rb = q[1];
+        const float4 ra = make_float4(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z), 0.0f);
+        if (g == 0u) {
+            const float3 p = unit_pos(bnd, xyz(ra));
+            upos[i] = make_float4(p.x, p.y, p.z, 0.0f);
+        }
+        store_group_inputs<(int)kEncodeGroups>(g, bnd, table, ra, rb, true, tiles + (size_t)tile * kActBytes, row);
     }
 }
 
@@ -493,7 +558,17 @@ __global__ void __launch_bounds__(256) k_cache_scatter(const float4* __restrict_
     }
 }
 
-// Forward + backward of every tile.
+// Forward + backward of every tile.  kTrainGroups threads share a sample, 64 / kTrainGroups
+// columns of every layer each.  What is left is the chain of ten layers' MMAs and barriers a
+// tile (7.9K cycles forward, 13.4K backward, of which the issuing thread waits 0.4K a layer
+// forward and 1K backward for the tensor core), one tile at a time in the shared memory.  The
+// 17K weight gradients go out 16 bytes at a time: as single words, each lane's in its own
+// sector and every block at the same addresses, they took 32 of 83 us for 65536 samples.
+#ifndef XR_TRAIN_GROUPS
+#define XR_TRAIN_GROUPS 2
+#endif
+constexpr int kTrainGroups = XR_TRAIN_GROUPS;
+constexpr uint32_t kCols = kWidth / kTrainGroups;
 // Shared memory (223,232 B): forward image, backward image, H_0..H_4, dZ,
 // dZ^T [128][128] (rows beyond the layer's outputs zero) and H^T [64][128] in
 // the padded transposed layout.
@@ -503,7 +578,7 @@ constexpr uint32_t kOffDZ = kOffX + 5 * kActBytes, kOffDZT = kOffDZ + kActBytes,
 constexpr uint32_t kTrainSmem = kOffHT + 8u * kTSbo;
 static_assert(kTrainSmem == 223232 && kTrainSmem <= 232448, "training shared memory layout");
 
-__global__ void __launch_bounds__(128, 1) k_cache_train(const uint4* __restrict__ rec, const uint32_t* __restrict__ perm,
+__global__ void __launch_bounds__(kTile* kTrainGroups, 1) k_cache_train(const uint4* __restrict__ rec, const uint32_t* __restrict__ perm,
                                                         const uint32_t* count_ptr,
                                                         uint32_t count_host, uint32_t cap, uint8_t* tiles,
                                                         const uint8_t* __restrict__ w_fwd,
@@ -519,6 +594,7 @@ __global__ void __launch_bounds__(128, 1) k_cache_train(const uint4* __restrict_
     __shared__ uint64_t bar;
     __shared__ uint32_t tslot;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    const uint32_t row = tid % kTile, col0 = tid / kTile * kCols;   // the thread's sample and its first column
     const uint32_t n = train_samples(count_ptr, count_host, cap);
     const uint32_t ntiles = n / kTile;
     if (blockIdx.x >= ntiles) return;
@@ -530,56 +606,56 @@ __global__ void __launch_bounds__(128, 1) k_cache_train(const uint4* __restrict_
     copy_image(sWb, w_bwd, kImageBytes);
     // rows 64..127 of dZ^T (row groups 8..15) stay zero -- the padding of the
     // M = 128 weight-gradient MMAs
-    for (uint32_t off = 8u * kTSbo + tid * 16u; off < 16u * kTSbo; off += 128u * 16u)
+    for (uint32_t off = 8u * kTSbo + tid * 16u; off < 16u * kTSbo; off += blockDim.x * 16u)
         *reinterpret_cast<uint4*>(sDZT + off) = make_uint4(0, 0, 0, 0);
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = tslot;
-    const uint32_t lane_addr = tmem + ((warp * 32u) << 16);
+    const uint32_t lane_addr = tmem + (((warp & 3u) * 32u) << 16);
     uint32_t phase = 0;
     bool ok = true, first = true;
     float loss = 0.0f;
 
     for (uint32_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-        const uint32_t i = tile * kTile + tid;
+        const uint32_t i = tile * kTile + row;
         uint8_t* tile_mem = tiles + (size_t)tile * kActBytes;
         {
-            // the tile's inputs, 8 x 16 B per thread; plain loads: this launch rewrites the tile below
-            uint4 q[kActBytes / 16 / kTile];
+            // the tile's inputs; plain loads: this launch rewrites the tile below
+            constexpr uint32_t kThreads = kTile * kTrainGroups, kEach = kActBytes / 16 / kThreads;
+            uint4 q[kEach];
 #pragma unroll
-            for (uint32_t k = 0; k < kActBytes / 16 / kTile; ++k)
-                q[k] = reinterpret_cast<const uint4*>(tile_mem)[k * kTile + tid];
+            for (uint32_t k = 0; k < kEach; ++k) q[k] = reinterpret_cast<const uint4*>(tile_mem)[k * kThreads + tid];
 #pragma unroll
-            for (uint32_t k = 0; k < kActBytes / 16 / kTile; ++k)
-                reinterpret_cast<uint4*>(sX)[k * kTile + tid] = q[k];
+            for (uint32_t k = 0; k < kEach; ++k) reinterpret_cast<uint4*>(sX)[k * kThreads + tid] = q[k];
         }
-        const uint4 rt = rec[(size_t)perm[i] * 3 + 2];
-        float v[kIn];
+        const uint4 rt = col0 == 0u ? rec[(size_t)perm[i] * 3 + 2] : make_uint4(0, 0, 0, 0);
+        float v[kCols];
         // ---- forward, keeping H_0..H_4 ----
         float y[16];
         for (int l = 0; l <= kHidden && ok; ++l) {
             publish();
             if (tid == 0) {
-                gemm(tmem, sX + l * kActBytes, sWf + l * kLayerBytes, 64u, l < kHidden ? 64u : 16u, 4u, false);
+                if (l < kHidden) gemm<64, 64>(tmem, sX + l * kActBytes, sWf + l * kLayerBytes);
+                else gemm<64, 16>(tmem, sX + l * kActBytes, sWf + l * kLayerBytes);
                 umma::commit(&bar);
             }
             ok = wait_mma(&bar, phase);
             if (!ok) break;
             if (l < kHidden) {
-                tmem_row64(lane_addr, v);
+                tmem_cols<kCols>(lane_addr + col0, v);
 #pragma unroll
-                for (int j = 0; j < kWidth; ++j) v[j] = fmaxf(v[j], 0.0f);
-                store_row<kIn>(sX + (l + 1) * kActBytes, tid, v);
-            } else {
+                for (int j = 0; j < kCols; ++j) v[j] = fmaxf(v[j], 0.0f);
+                store_cols<kCols>(sX + (l + 1) * kActBytes, row, col0, v);
+            } else if (col0 == 0u) {
                 umma::tmem_ld16(lane_addr, y);
                 umma::tmem_wait_ld();
             }
         }
         if (!ok) break;
         // ---- loss and output gradient ----
-        float dz[kWidth];
-        {
+        if (col0 == 0u) {
+            float dz[16];
             const float t[3] = {__uint_as_float(rt.x), __uint_as_float(rt.y), __uint_as_float(rt.z)};
 #pragma unroll
             for (int c = 0; c < 16; ++c) dz[c] = 0.0f;
@@ -590,44 +666,45 @@ __global__ void __launch_bounds__(128, 1) k_cache_train(const uint4* __restrict_
                 loss += d * d / den * inv_count;
                 dz[c] = 2.0f * d / den * inv_count;
             }
+            store_row<16>(sDZ, row, dz);
+            store_col_t<16>(sDZT, 0u, row, dz);
         }
-        store_row<16>(sDZ, tid, dz);
-        store_col_t<16>(sDZT, tid, dz);
         // rows 16..63 of dZ^T (row groups 2..7): zero -- the previous tile's hidden
         // layers left values there
-        for (uint32_t off = 2u * kTSbo + tid * 16u; off < 8u * kTSbo; off += 128u * 16u)
+        for (uint32_t off = 2u * kTSbo + tid * 16u; off < 8u * kTSbo; off += blockDim.x * 16u)
             *reinterpret_cast<uint4*>(sDZT + off) = make_uint4(0, 0, 0, 0);
         // ---- backward: layer 4 .. 0 ----
         for (int l = kHidden; l >= 0 && ok; --l) {
             // H_l^T from this thread's own row of H_l
-            load_row64(sX + l * kActBytes, tid, v);
-            store_col_t<64>(sHT, tid, v);
+            load_cols<kCols>(sX + l * kActBytes, row, col0, v);
+            store_col_t<kCols>(sHT, col0, row, v);
             publish();
             if (tid == 0) {
-                const uint32_t K = l == kHidden ? 16u : 64u;
-                gemm(tmem, sDZ, sWb + l * kLayerBytes, K, 64u, K / 16u, false);                  // dX = dZ W_l
-                gemm_t(tmem + 64u + 64u * (uint32_t)l, sDZT, sHT, 64u, !first);                // dW_l += dZ^T H_l
+                if (l == kHidden) gemm<16, 64>(tmem, sDZ, sWb + l * kLayerBytes);   // dX = dZ W_l
+                else gemm<64, 64>(tmem, sDZ, sWb + l * kLayerBytes);
+                gemm_t(tmem + 64u + 64u * (uint32_t)l, sDZT, sHT, !first);           // dW_l += dZ^T H_l
                 umma::commit(&bar);
             }
             ok = wait_mma(&bar, phase);
             if (!ok) break;
-            float dx[kWidth];
-            tmem_row64(lane_addr, dx);
+            float dx[kCols];
+            tmem_cols<kCols>(lane_addr + col0, dx);
             if (l > 0) {
                 // dZ_l = dH_l * relu'(Z_l), with Z_l > 0 exactly where this thread's row of H_l (in v) is
 #pragma unroll
-                for (int j = 0; j < kWidth; ++j) dz[j] = v[j] > 0.0f ? dx[j] : 0.0f;
-                store_row<kIn>(sDZ, tid, dz);
+                for (int j = 0; j < kCols; ++j) dx[j] = v[j] > 0.0f ? dx[j] : 0.0f;
+                store_cols<kCols>(sDZ, row, col0, dx);
                 // the bf16-rounded values of dz, as the MMA will see them
 #pragma unroll
-                for (int j = 0; j < kWidth; ++j) dz[j] = umma::bf16_value(umma::bf16_bits(dz[j]));
-                store_col_t<64>(sDZT, tid, dz);
-            } else {
+                for (int j = 0; j < kCols; ++j) dx[j] = umma::bf16_value(umma::bf16_bits(dx[j]));
+                store_col_t<kCols>(sDZT, col0, row, dx);
+            } else if (col0 < 2u * kLevels) {
                 // gradients of the 32 encoding features, feature-major over the tile's inputs (every
                 // thread's loads of the tile completed before the first barrier of this tile)
-                float* g = reinterpret_cast<float*>(tile_mem) + tid;
+                float* g = reinterpret_cast<float*>(tile_mem) + row;
 #pragma unroll
-                for (int j = 0; j < 2 * kLevels; ++j) g[j * kTile] = dx[j];
+                for (uint32_t j = 0; j < kCols; ++j)
+                    if (col0 + j < 2u * kLevels) g[(col0 + j) * kTile] = dx[j];
             }
         }
         first = false;
@@ -635,18 +712,20 @@ __global__ void __launch_bounds__(128, 1) k_cache_train(const uint4* __restrict_
     // loss (mean over the batch)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xFFFFFFFFu, loss, o);
-    if (lane == 0 && ok) atomicAdd(loss_acc, loss);
-    // weight gradients: rows 0..63 live in warps 0 and 1
-    if (ok && !first && warp < 2) {
+    if (lane == 0 && col0 == 0u && ok) atomicAdd(loss_acc, loss);
+    // weight gradients: rows 0..63 live in the first two warps of each group
+    if (ok && !first && (warp & 3u) < 2u) {
         for (int l = 0; l <= kHidden; ++l) {
             const uint32_t rows = l < kHidden ? 64u : 16u;
-            for (uint32_t c = 0; c < 64u; c += 16u) {
+            for (uint32_t c = col0; c < col0 + kCols; c += 16u) {
                 float g[16];
                 umma::tmem_ld16(lane_addr + 64u + 64u * (uint32_t)l + c, g);
                 umma::tmem_wait_ld();
-                if (tid < rows) {
+                if (row < rows) {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) atomicAdd(mlp_grad + l * 4096 + tid * 64u + c + j, g[j]);
+                    for (int j = 0; j < 16; j += 4)
+                        red_add4(reinterpret_cast<float2*>(mlp_grad + l * 4096 + row * 64u + c + j), g[j], g[j + 1],
+                                 g[j + 2], g[j + 3]);
                 }
             }
         }
@@ -863,17 +942,17 @@ void launch_cache_pack(const XrCacheSample* s, uint32_t n, uint4* rec, uint32_t 
 void launch_cache_infer(CacheState& cs, const uint4* rec, const uint32_t* count_ptr, uint32_t count_host,
                         float* out3, float4* cand_b, uint32_t* err, int sm_count, cudaStream_t st) {
     const uint32_t smem = kImageBytes + kActBytes;
-    uint32_t grid = (uint32_t)sm_count * 4u;
+    uint32_t grid = (uint32_t)(sm_count * kInferBlocks);
     if (!count_ptr) {
         const uint32_t tiles = (count_host + kTile - 1u) / kTile;
         if (tiles == 0) return;
         if (tiles < grid) grid = tiles;
     }
     if (cand_b)
-        k_cache_infer<1><<<grid, 128, smem, st>>>(rec, count_ptr, count_host, bounds_of(cs), cs.table, cs.w_fwd,
+        k_cache_infer<1><<<grid, kTile * kInferGroups, smem, st>>>(rec, count_ptr, count_host, bounds_of(cs), cs.table, cs.w_fwd,
                                                   nullptr, cand_b, err);
     else
-        k_cache_infer<0><<<grid, 128, smem, st>>>(rec, count_ptr, count_host, bounds_of(cs), cs.table, cs.w_fwd,
+        k_cache_infer<0><<<grid, kTile * kInferGroups, smem, st>>>(rec, count_ptr, count_host, bounds_of(cs), cs.table, cs.w_fwd,
                                                   out3, nullptr, err);
 }
 
@@ -932,7 +1011,7 @@ void launch_cache_grad_stage(CacheState& cs, const uint4* rec, const uint32_t* c
     const uint32_t wide = (uint32_t)sm_count * 8u;
     const uint32_t* perm = cs.order + 3 * (size_t)cs.train_cap;   // the sort's result (second value array)
     const float4* upos = reinterpret_cast<const float4*>(cs.order + 4 * (size_t)cs.train_cap);
-    k_cache_train<<<grid, 128, kTrainSmem, st>>>(rec, perm, count_ptr, count_host, cap, cs.tiles, cs.w_fwd, cs.w_bwd,
+    k_cache_train<<<grid, kTile * kTrainGroups, kTrainSmem, st>>>(rec, perm, count_ptr, count_host, cap, cs.tiles, cs.w_fwd, cs.w_bwd,
                                                  cs.mlp_grad, cs.loss, err);
     k_cache_scatter<<<wide, 256, 0, st>>>(upos, count_ptr, count_host, cap, reinterpret_cast<const float*>(cs.tiles),
                                           reinterpret_cast<float2*>(cs.grid_grad), err);

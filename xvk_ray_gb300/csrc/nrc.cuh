@@ -126,44 +126,40 @@ __device__ __forceinline__ float3 unit_pos(const Bounds& b, float3 x) {
     return p;
 }
 
-// The 64 network inputs of one record, as float values (rounded to bfloat16 by
-// the caller when staged for the tensor core).
-__device__ __forceinline__ void network_inputs(const Bounds& bnd, const __half2* __restrict__ table, float4 ra,
-                                               uint4 rb, float* v) {
-    const float3 p = unit_pos(bnd, xyz(ra));
+// The two features of level l at the unit position p.
+__device__ __forceinline__ void level_features(int l, float3 p, const __half2* __restrict__ table, float* v) {
+    LevelCorners c;
+    level_corners(l, p, c);
+    __half2 t[8];
 #pragma unroll
-    for (int l = 0; l < kLevels; ++l) {
-        LevelCorners c;
-        level_corners(l, p, c);
-        __half2 t[8];
+    for (int k = 0; k < 8; ++k) t[k] = __ldg(table + (size_t)l * kT + c.idx[k]);
+    float a0 = 0.0f, a1 = 0.0f;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) t[k] = __ldg(table + (size_t)l * kT + c.idx[k]);
-        float a0 = 0.0f, a1 = 0.0f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const float2 tv = __half22float2(t[k]);
-            a0 = a0 + c.w[k] * tv.x;
-            a1 = a1 + c.w[k] * tv.y;
-        }
-        v[2 * l] = a0;
-        v[2 * l + 1] = a1;
+    for (int k = 0; k < 8; ++k) {
+        const float2 tv = __half22float2(t[k]);
+        a0 = a0 + c.w[k] * tv.x;
+        a1 = a1 + c.w[k] * tv.y;
     }
+    v[0] = a0;
+    v[1] = a1;
+}
+
+// The 16 inputs after the encoding's features.
+__device__ __forceinline__ void other_inputs(uint4 rb, float* v) {
     const float3 n = oct_decode(rb.x, 16), wo = oct_decode(rb.y, 16);
     const float ndw = dot(n, wo);
     const float3 refl = n * (2.0f * ndw) - wo;
     const uint32_t kind = rb.z >> 24;
-    v[32] = n.x; v[33] = n.y; v[34] = n.z;
-    v[35] = wo.x; v[36] = wo.y; v[37] = wo.z;
-    v[38] = refl.x; v[39] = refl.y; v[40] = refl.z;
-    v[41] = (float)(rb.z & 255u) / 255.0f;
-    v[42] = (float)((rb.z >> 8) & 255u) / 255.0f;
-    v[43] = (float)((rb.z >> 16) & 255u) / 255.0f;
-    v[44] = __uint_as_float(rb.w);
-    v[45] = kind == 1u ? 1.0f : 0.0f;
-    v[46] = kind == 5u ? 1.0f : 0.0f;
-    v[47] = 1.0f;
-#pragma unroll
-    for (int j = 48; j < kIn; ++j) v[j] = 0.0f;
+    v[0] = n.x; v[1] = n.y; v[2] = n.z;
+    v[3] = wo.x; v[4] = wo.y; v[5] = wo.z;
+    v[6] = refl.x; v[7] = refl.y; v[8] = refl.z;
+    v[9] = (float)(rb.z & 255u) / 255.0f;
+    v[10] = (float)((rb.z >> 8) & 255u) / 255.0f;
+    v[11] = (float)((rb.z >> 16) & 255u) / 255.0f;
+    v[12] = __uint_as_float(rb.w);
+    v[13] = kind == 1u ? 1.0f : 0.0f;
+    v[14] = kind == 5u ? 1.0f : 0.0f;
+    v[15] = 1.0f;
 }
 
 }  // namespace nrc
