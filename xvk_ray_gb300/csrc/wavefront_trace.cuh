@@ -509,8 +509,14 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
         const bool enter = INST && !in_blas && tg_mask != 0u;
         if (INST && (n_run < kMinRunning || __popc(__ballot_sync(FULL, enter)) >= (int)kEnterMin) && enter) {
             const uint4 w1 = __ldg(reinterpret_cast<const uint4*>(sc.tlas_nodes + tg_base) + 1);
-            const uint32_t slot = w1.y + __popc(w1.z & (tg_mask - 1u) & ~tg_mask);
-            tg_mask &= tg_mask - 1u;
+            // the instances of the node in the order its children are visited, nearest octant first
+            uint32_t m = tg_mask, part;
+            if ((part = m & ((flip & 4u) ? 0xFFF000u : 0x000FFFu))) m = part;
+            if ((part = m & ((flip & 2u) ? 0xFC0FC0u : 0x03F03Fu))) m = part;
+            if ((part = m & ((flip & 1u) ? 0xE38E38u : 0x1C71C7u))) m = part;
+            m &= 0u - m;
+            const uint32_t slot = w1.y + __popc(w1.z & (m - 1u));
+            tg_mask ^= m;
             if (slot >= sc.n_inst_slots || sp + 3u > (uint32_t)kStackSize) {
                 overflow();
                 tg_mask = 0u;
