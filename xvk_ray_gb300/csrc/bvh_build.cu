@@ -1246,22 +1246,42 @@ xr_status build_wide(Context* ctx, WideBuild& B) {
     const char* coll = getenv("XR_BVH_COLLAPSE");   // greedy: the area-greedy widening instead of the SAH decisions
     const bool sah = n > 1 && !(coll && strcmp(coll, "greedy") == 0);
     const uint32_t np = ploc ? n : 0u, nd = sah ? nint : 0u;
-    {   // one stream-ordered allocation holds all scratch
+    {   // One stream-ordered allocation holds all scratch.  Mapping and returning it takes a
+        // microsecond or more a megabyte, a fifth of a 1M-triangle build, so arrays share memory
+        // where one's last use comes before the other's first, in stream order: sort and clustering
+        // with what follows them, the costs of the SAH decisions with the collapse (328 -> 212 bytes
+        // a primitive).
         struct Item { void** dst; size_t bytes; };
         std::vector<Item> items;
         auto add = [&](auto** dst, size_t count) { items.push_back({(void**)dst, count * sizeof(**dst)}); };
-        add(&tlo, n); add(&thi, n); add(&k0, n); add(&k1, n); add(&v0, n); add(&v1, n);
-        add(&hist, 256 * ((size_t)nblk + 1)); add(&left, nint); add(&right, nint); add(&pint, nint); add(&pleaf, n);
-        add(&flags, (size_t)nint + 1); add(&range, nint); add(&nlo, nint); add(&nhi, nint);
-        add(&ta, n); add(&tb, n); add(&wa, n); add(&wb, n); add(&words, 1); add(&nodes_tmp, nint);
-        add(&clo, np); add(&chi, np); add(&olo, np); add(&ohi, np); add(&nn, np); add(&sums, np / 1024 + 1);
-        add(&sah_cost, 8 * (size_t)nd); add(&sah_dec, kDecStride * (size_t)nd); add(&sah_flags, (size_t)nd + 1);
-        auto up = [](size_t v) { return (v + 255u) & ~size_t(255u); };
-        size_t total = 0;
-        for (const Item& it : items) total += up(it.bytes);
-        if ((s = pool_alloc_bytes(ctx, &scratch, total, "bvh scratch"))) goto done;
-        size_t off = 0;
-        for (const Item& it : items) { *it.dst = (char*)scratch + off; off += up(it.bytes); }
+        // the offset behind the items added since the last call, laid out from `off`
+        char* base = nullptr;
+        auto place = [&](size_t off) {
+            for (const Item& it : items) {
+                if (base) *it.dst = base + off;
+                off += (it.bytes + 255u) & ~size_t(255u);
+            }
+            items.clear();
+            return off;
+        };
+        auto layout = [&]() {
+            add(&tlo, n); add(&thi, n); add(&v0, n); add(&left, nint); add(&right, nint); add(&pint, nint); add(&pleaf, n);
+            add(&flags, (size_t)nint + 1); add(&range, nint); add(&nlo, nint); add(&nhi, nint); add(&words, 1);
+            const size_t all = place(0);
+            add(&k0, n); add(&k1, n); add(&v1, n); add(&hist, 256 * ((size_t)nblk + 1));
+            add(&clo, np); add(&chi, np); add(&olo, np); add(&ohi, np); add(&nn, np); add(&sums, np / 1024 + 1);
+            const size_t tree = place(all);
+            add(&sah_dec, kDecStride * (size_t)nd); add(&sah_flags, (size_t)nd + 1);
+            const size_t decided = place(all);
+            add(&sah_cost, 8 * (size_t)nd);
+            const size_t deciding = place(decided);
+            add(&ta, n); add(&tb, n); add(&wa, n); add(&wb, n); add(&nodes_tmp, nint);
+            const size_t collapse = place(decided);
+            return std::max(tree, std::max(deciding, collapse));
+        };
+        if ((s = pool_alloc_bytes(ctx, &scratch, layout(), "bvh scratch"))) goto done;
+        base = (char*)scratch;
+        layout();
     }
     if (!B.slots_into && (s = dalloc(ctx, &B.slots, (size_t)slot_words * n))) goto done;
     if (B.slots_into) B.slots = B.slots_into;
