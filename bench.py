@@ -798,7 +798,7 @@ def run_batch(args):
         "ms_per_frame_direct_launches": round(ms_direct, 4),
         "graph_speedup": round(ms_direct / ms_graph, 4),
         "tuning": {"trace_ctas_per_sm": tuning.trace_ctas_per_sm, "shade_ctas_per_sm": tuning.shade_ctas_per_sm,
-                   "refill_min": tuning.refill_min or "default (8)", "postpone_below": tuning.postpone_below or "default (32, with instances 16)",
+                   "refill_min": tuning.refill_min or "default (8; 20 below 12288 nodes)", "postpone_below": tuning.postpone_below or "default (32, with instances 16)",
                    "ray_bundle": ["8x4", "16x2", "4x8"][tuning.ray_bundle],
                    "temporal_block": tuning.temporal_block or "default (64)",
                    "spatial_block": tuning.spatial_block or "default (128)",

@@ -342,7 +342,7 @@ typedef struct XrTuning {
     float ms_default;            /* xr_autotune: the all-defaults configuration */
     uint32_t configs_tried;
     /* ray queues of the persistent traversal: a warp refills from its queue once this many
-       lanes are idle (default 8), and tests triangles once this many are queued (default 32, with instances 16) */
+       lanes are idle (default 8, in trees of fewer than 12288 nodes 20), and tests triangles once this many are queued (default 32, with instances 16) */
     uint32_t refill_min, postpone_below;
     uint32_t ray_bundle;         /* camera rays of a 16 x 8 tile per warp: 0 8x4 blocks (default), 1 16x2 rows, 2 4x8 */
     uint32_t temporal_block;     /* threads per block of the temporal pass: 32, 64 (default), 128, 256 */

@@ -157,7 +157,7 @@ __device__ __forceinline__ void tmem_cols(uint32_t taddr, float* v) {
 // activations and the rest of the inputs are split between them.  The kernel waits for the
 // table's gathers (L1 hits half of them) and, layer by layer, for its own block: it wants warps
 // and L1.  Two threads a sample and three blocks an SM (24 warps, 156 of 256 KB shared) take
-// 99 us for the 1.3M queries of a 1080p frame and 40 for 65536; one thread and four blocks
+// 97 us for the 0.44M queries of a 1080p frame and 40 for 65536; one thread and four blocks
 // (213 KB shared, a second wave) 153 and 77, two and four 161 and 80, two and two 116 and 38,
 // four and two 116 and 41, two and three with the largest carve-out 159 and 75.
 #ifndef XR_INFER_GROUPS
