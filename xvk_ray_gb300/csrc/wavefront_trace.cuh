@@ -251,8 +251,10 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
         }
         if (e.y & 0xFFu) take_child(e, tail);
     };
-    // Rays (their lanes) with a queued test.
+    // Rays (their lanes) with a queued test.  The entries are other lanes' writes, and a vote
+    // orders no memory: without the barrier a ray could be stored before its last test.
     auto queued_rays = [&]() {
+        __syncwarp();
         uint32_t m = 0u;
         for (uint32_t i = 0; i < q_count; i += 32u)
             m |= __reduce_or_sync(FULL, i + lane < q_count ? 1u << sh.q_lane[(q_head + i + lane) & (kTriQueue - 1u)] : 0u);
@@ -309,7 +311,9 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
         }
         if (!ANY) h_t = sh.t[ray];
         else if (sh.prim[ray] >= 0) { cur = kInvalid; tg_mask = 0u; sp = sb = 0; }   // occluded: nothing left to visit
-        if (INST) pending = queued_rays();
+        // the rays, records and queue entries read above are written again from here on
+        if (INST) pending = queued_rays();   // its barrier comes first
+        else __syncwarp();
     };
 
     // One round: finished rays out and new ones in, a node per lane, the tests it gave.
