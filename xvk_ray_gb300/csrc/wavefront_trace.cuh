@@ -211,9 +211,10 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
         }
     };
     // A group whose nearest child starts beyond the closest hit has nothing left to find:
-    // the bound is below every child's entry, and the margin is the box test's own.
+    // the bound is below every child's entry, and the margin is the box test's own.  A bound
+    // of 0 stands for any entry below, so a hit behind the origin drops no group for it.
     auto beyond = [&](uint2 e) {
-        return __uint_as_float(e.y & 0xFFFF0000u) > (h_t * (1.0f + 1e-6f) + 1e-30f) * (1.0f + 2e-6f);
+        return __uint_as_float(e.y & 0xFFFF0000u) > fmaxf((h_t * (1.0f + 1e-6f) + 1e-30f) * (1.0f + 2e-6f), 0.0f);
     };
     // The whole ray's start: at the top-level root, or at the root of its scene.
     auto start_ray = [&](uint32_t root) {
@@ -489,7 +490,8 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
                 if (NEAR && ih) {
                     // The nearest hit box, when it is an internal child, is visited next and the
                     // second nearest bounds the rest from below; else the first child in octant
-                    // order, and the nearest box is the bound.
+                    // order, and the nearest box is the bound.  (Entries behind the origin are
+                    // ordered backwards as integers: any of them may come first, and the bound is 0.)
                     const uint32_t s1 = (uint32_t)near1 & 7u;
                     const bool is_node = (w1.z >> (24u + s1)) & 1u;
                     found.y |= (uint32_t)max(is_node ? near2 : near1, 0) & 0xFFFF0000u;
