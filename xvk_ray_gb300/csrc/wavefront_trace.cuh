@@ -86,14 +86,6 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
     return r;
 }
 
-// Reciprocal within one ulp: enough for the box test, whose far planes are widened by
-// a relative 2e-6.
-__device__ __forceinline__ float rcp_box(float x) {
-    float r;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-
 // Per-warp working set of the traversal in shared memory: the queue of triangle tests,
 // and per lane its ray as the triangle test wants it and the closest hit so far.
 constexpr uint32_t kTriQueue = 64;
@@ -183,11 +175,13 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
     // departs from the true one by at most kMinDir * t, far inside the slack of the stored
     // boxes, so no box holding a hit is culled; the triangle test uses the true direction.
     // The sign bits select the near planes (so that -0 picks the same planes as its
-    // infinite reciprocal).
+    // infinite reciprocal).  The divisions are correctly rounded: rcp.approx, within an ulp,
+    // would save 2% of the dynamic world's frame and 0.6% of one level's, but the planes'
+    // constants then start from a less exact operand.
     auto set_dir = [&](float3 d) {
-        idx = rcp_box(copysignf(fmaxf(fabsf(d.x), kMinDir), d.x));
-        idy = rcp_box(copysignf(fmaxf(fabsf(d.y), kMinDir), d.y));
-        idz = rcp_box(copysignf(fmaxf(fabsf(d.z), kMinDir), d.z));
+        idx = 1.0f / copysignf(fmaxf(fabsf(d.x), kMinDir), d.x);
+        idy = 1.0f / copysignf(fmaxf(fabsf(d.y), kMinDir), d.y);
+        idz = 1.0f / copysignf(fmaxf(fabsf(d.z), kMinDir), d.z);
         flip = (__float_as_uint(d.x) >> 31) | ((__float_as_uint(d.y) >> 31) << 1) | ((__float_as_uint(d.z) >> 31) << 2);
     };
     // The lane's ray as every lane's triangle test reads it.
