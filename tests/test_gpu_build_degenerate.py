@@ -1,0 +1,83 @@
+"""BVH builds over primitives without area, the smallest inputs and boxes that coincide:
+the build ends in a tree of bounded depth, and hits are the oracle's bit for bit."""
+import numpy as np
+import pytest
+
+import xvk_ray_gb300 as xr
+from oracle import binding as ob
+from tests.helpers import affine, box_scene, random_rays
+from tests.test_gpu_traversal_queue import _rays, _soup
+
+pytestmark = pytest.mark.gpu
+
+
+def _with_triangles(extra):
+    """The Cornell box behind the triangles `extra` (k x 3 x 3)."""
+    base = xr.Scene.cornell()
+    k = len(extra)
+    v = np.zeros((3 * k, 9), np.float32)
+    v[:, :3] = np.asarray(extra, np.float32).reshape(-1, 3)
+    v[:, 4] = 1.0
+    v[:, 8] = base.vertices[0, 8]
+    idx = np.concatenate([np.arange(3 * k, dtype=np.uint32), base.global_indices().astype(np.uint32) + 3 * k])
+    return xr.Scene(np.concatenate([v, base.vertices]), idx, base.materials, np.zeros((1, 2), np.uint32), base.camera)
+
+
+def _alone(tri):
+    """A scene of these triangles alone."""
+    v = np.zeros((3 * len(tri), 9), np.float32)
+    v[:, :3] = np.asarray(tri, np.float32).reshape(-1, 3)
+    v[:, 4] = 1.0
+    base = xr.Scene.cornell()
+    return xr.Scene(v, np.arange(3 * len(tri), dtype=np.uint32), base.materials[:1].copy(), np.zeros((1, 2), np.uint32),
+                    base.camera)
+
+
+def _check(scene, rays, max_depth):
+    op, ot, obary = ob.OracleScene.from_scene(scene).trace(rays)
+    hit = op >= 0
+    with xr.Renderer(8, 8) as r:
+        r.upload_scene(scene)
+        r.build_bvh()
+        gp, gt, gb = r.trace(rays)
+        st = r.stats()
+    assert st.error_flags == 0 and st.bvh_triangles == scene.n_triangles
+    assert st.bvh_depth <= max_depth
+    assert np.array_equal(gp, op)
+    assert np.array_equal(gt[hit].view(np.uint32), ot[hit].view(np.uint32))
+    assert np.array_equal(gb[hit].view(np.uint32), obary[hit].view(np.uint32))
+
+
+@pytest.mark.parametrize("builder", ["ploc", "lbvh"])
+@pytest.mark.parametrize("n", [4, 5, 8])
+@pytest.mark.parametrize("kind", ["point", "line"])
+def test_triangles_without_area(kind, n, builder, monkeypatch):
+    """Points and axis-parallel segments: every SAH cost of their subtree is 0."""
+    monkeypatch.setenv("XR_BVH_BUILDER", builder)
+    tri = np.full((n, 3, 3), 0.5)
+    if kind == "line":
+        tri[:, :, 0] = np.arange(3 * n).reshape(n, 3) * 0.01
+    rays = random_rays(np.random.default_rng(n), 2000, [-1, 0, -1], [1, 2, 1])
+    _check(_alone(tri), rays, n)
+    _check(_with_triangles(tri), rays, n + 4)
+
+
+@pytest.mark.parametrize("builder", ["ploc", "karras"])
+def test_instances_of_empty_scenes_at_one_point(builder, monkeypatch):
+    """Instances of a scene without triangles are point boxes at their origin."""
+    monkeypatch.setenv("XR_TLAS_BUILDER", builder)
+    rng = np.random.default_rng(3)
+    scene = box_scene(rng, 12, 2.0)
+    empty = xr.Scene(scene.vertices, scene.indices[:0].copy(), scene.materials, scene.ranges, scene.camera)
+    inst = [(1, affine(np.eye(3), [1, 2, 3]))] * 5 + [(0, affine(np.eye(3), [0, 0, 0]))]
+    rays = random_rays(rng, 2000, -4, 4)
+    world = ob.OracleWorld([ob.OracleScene.from_scene(s) for s in (scene, empty)])
+    world.set_instances(inst)
+    c = world.trace_instanced(rays)
+    with xr.Renderer(8, 8) as r:
+        r.upload_scenes([scene, empty])
+        r.set_instances(inst)
+        g = r.trace_instanced(rays)
+        assert r.stats().error_flags == 0
+    for x, y in zip(g, c):
+        assert np.array_equal(np.asarray(x).view(np.uint32), np.asarray(y).view(np.uint32))

@@ -393,13 +393,15 @@ __device__ __forceinline__ int ceil_log2f(float v) {   // smallest e with 2^e >=
 //                    wide node: A(n) cn + min_{j=2..8} D(n, j)),
 //   cost(n, i) = min(cost(n, i - 1), D(n, i)),  D(n, i) = min_k cost(l, k) + cost(r, i - k);
 // a primitive costs A ct for every i.  Computed bottom-up (the second thread to
-// reach a node evaluates it); the decisions -- leaf or wide node, the best j, and
-// per i the split k (0: i - 1 children suffice) -- drive the top-down collapse.
+// reach a node evaluates it); the decisions -- the best j with its split, and per i the
+// split k (0: i - 1 children suffice) -- drive the top-down collapse.  A wide node's own
+// subtree is always split: where every cost is 0 or infinite (primitives without area, or
+// too large for it) no split is ever cheaper, and the node would be its own only child.
 #ifndef XR_SAH_TRI
 #define XR_SAH_TRI 1.2f
 #endif
 constexpr float kSahNode = 1.0f, kSahTri = XR_SAH_TRI;
-constexpr uint32_t kDecStride = 16;   // bytes per binary node: [0] leaf?, [1] j*, [i] split of i (2..8)
+constexpr uint32_t kDecStride = 16;   // bytes per binary node: [0] split of j*, [1] j*, [i] split of i (2..8)
 
 __global__ void k_parents(uint32_t nint, const uint32_t* __restrict__ left, const uint32_t* __restrict__ right,
                           uint32_t* __restrict__ parent_int, uint32_t* __restrict__ parent_leaf, const uint32_t* made) {
@@ -454,11 +456,11 @@ __global__ void k_sah_dp(int n, const uint32_t* __restrict__ left, const uint32_
                 if (v < D[i]) { D[i] = v; ks[i] = (uint32_t)k; }
             }
         }
-        uint32_t jstar = 2u;
+        uint32_t jstar = 2u, kstar = ks[2];
         float dbest = D[2];
 #pragma unroll
         for (int i = 3; i <= 8; i++)
-            if (D[i] < dbest) { dbest = D[i]; jstar = (uint32_t)i; }
+            if (D[i] < dbest) { dbest = D[i]; jstar = (uint32_t)i; kstar = ks[i]; }
         const float4 lo = __ldcg(nlo + node), hi = __ldcg(nhi + node);
         const float dx = hi.x - lo.x, dy = hi.y - lo.y, dz = hi.z - lo.z;
         const float A = dx * dy + dy * dz + dz * dx;
@@ -466,7 +468,7 @@ __global__ void k_sah_dp(int n, const uint32_t* __restrict__ left, const uint32_
         const float c_leaf = cnt <= 3u ? A * kSahTri * (float)cnt : INFINITY;
         const float c_int = A * kSahNode + dbest;
         // 16 decision bytes and 8 costs, each written as whole words
-        uint32_t d[4] = {(c_leaf <= c_int ? 1u : 0u) | (jstar << 8), 0u, 0u, 0u};
+        uint32_t d[4] = {kstar | (jstar << 8), 0u, 0u, 0u};
         float c[9];
         c[1] = fminf(c_leaf, c_int);
 #pragma unroll
@@ -567,7 +569,7 @@ __global__ void __launch_bounds__(128) k_collapse(CollapseArgs a, uint32_t level
                 const bool open = i > 1u && !(x & kLeafBit);
                 uint32_t k = 0u, r = 0u, l = 0u;
                 if (open) {
-                    k = a.dec[(size_t)kDecStride * x + i];
+                    k = a.dec[(size_t)kDecStride * x + (x == bref ? 0u : i)];
                     l = a.left[x];
                     r = a.right[x];
                 }
