@@ -81,3 +81,46 @@ def test_instances_of_empty_scenes_at_one_point(builder, monkeypatch):
         assert r.stats().error_flags == 0
     for x, y in zip(g, c):
         assert np.array_equal(np.asarray(x).view(np.uint32), np.asarray(y).view(np.uint32))
+
+
+def _log2(n):
+    return max(int(np.ceil(np.log2(n))), 1)
+
+
+@pytest.mark.parametrize("builder", ["ploc", "lbvh"])
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 65, 200, 2047, 2049, 3000])
+@pytest.mark.parametrize("kind", ["one", "point", "row"])
+def test_boxes_that_tie(kind, n, builder, monkeypatch):
+    """One triangle many times, one point many times, a row of equal triangles: merged boxes
+    of equal area everywhere, and still a tree no deeper than a balanced binary one."""
+    monkeypatch.setenv("XR_BVH_BUILDER", builder)
+    tri = np.tile(np.array([[[-0.5, -0.5, 0.0], [0.5, -0.5, 0.25], [0.0, 0.5, 0.0]]]), (n, 1, 1))
+    if kind == "point":
+        tri[:] = 0.25
+    if kind == "row":
+        tri[:, :, 0] += (np.arange(n)[:, None] - n // 2) * 1.25
+    _check(_alone(tri), _rays(300, n), _log2(n))
+
+
+@pytest.mark.parametrize("n", [32, 256, 1500, 2100])
+@pytest.mark.parametrize("kind", ["one", "row"])
+def test_instances_whose_boxes_tie(kind, n, monkeypatch):
+    """Instances spawned at one place or set up in a row, with the clustering builder."""
+    monkeypatch.setenv("XR_TLAS_BUILDER", "ploc")
+    rng = np.random.default_rng(n)
+    scene = box_scene(rng, 6, 2.0)
+    inst = [(0, affine(np.eye(3), [8.0 * k if kind == "row" else 0.5, 0, 0])) for k in range(n)]
+    _check_world([scene], inst, random_rays(rng, 300, [-4, -4, -4], [60 if kind == "row" else 4, 4, 4]))
+
+
+def _check_world(scenes, inst, rays):
+    world = ob.OracleWorld([ob.OracleScene.from_scene(s) for s in scenes])
+    world.set_instances(inst)
+    c = world.trace_instanced(rays)
+    with xr.Renderer(8, 8) as r:
+        r.upload_scenes(scenes)
+        r.set_instances(inst)
+        g = r.trace_instanced(rays)
+        assert r.stats().error_flags == 0
+    for x, y in zip(g, c):
+        assert np.array_equal(np.asarray(x).view(np.uint32), np.asarray(y).view(np.uint32))

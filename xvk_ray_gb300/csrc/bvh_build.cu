@@ -919,10 +919,13 @@ __global__ void k_esc(const uint4* __restrict__ tri_idx, const float4* __restric
 // ---- PLOC: Meister and Bittner, "Parallel Locally-Ordered Clustering for
 // Bounding Volume Hierarchy Construction" (TVCG 2018).  Clusters stay in
 // Morton order; each finds the cluster within +-kPlocRadius positions whose
-// merged box has the smallest surface area (ties by the pair's indices, so the
-// globally best pair is always mutual and every round merges), mutual pairs
-// merge into a new internal node at the lower position, the array is
-// compacted, and rounds repeat until one cluster is left.
+// merged box has the smallest surface area, mutual pairs merge into a new
+// internal node at the lower position, the array is compacted, and rounds repeat
+// until one cluster is left.  Of equal areas the partner (positions 2k and 2k + 1)
+// comes first, then the pairs by their indices: the globally best pair is always
+// mutual, so every round merges, and boxes that coincide or stand in a regular row
+// halve in a round (by the indices alone 256 equal boxes merged one pair a round into
+// a chain of 255 nodes, a row of 256 took 135 rounds; 8 and 8).
 #ifndef XR_PLOC_RADIUS
 #define XR_PLOC_RADIUS 64
 #endif
@@ -951,9 +954,9 @@ __device__ __forceinline__ float merged_area(float4 alo, float4 ahi, float4 blo,
 // What stands for a position outside the array: its merged area is infinite, so it never wins.
 __device__ __forceinline__ float4 nowhere(float s) { return make_float4(s * INFINITY, s * INFINITY, s * INFINITY, 0.0f); }
 
-// Nearest neighbours.  Candidates are taken in ascending order with a strict comparison:
-// of equal areas the lowest position wins, which orders pairs by area, lower index, upper
-// index.  A thread searches for two adjacent clusters, so that each candidate read from
+// Nearest neighbours.  The partner is taken first, then the candidates in ascending order
+// with a strict comparison: of equal areas the partner wins, then the lowest position, which
+// orders the other pairs by area, lower index, upper index.  A thread searches for two adjacent clusters, so that each candidate read from
 // shared memory serves two (reading it was the bound: 128 x 32 B per cluster); even and
 // odd positions are stored apart, so that the threads' reads are consecutive.  SPLIT > 1:
 // that many lanes share a pair's candidates, for counts that leave the chip idle and the
@@ -976,28 +979,30 @@ __global__ void __launch_bounds__(kPlocBlock) k_ploc_nn(const uint32_t* n_ptr, c
     __syncthreads();
     const int t = threadIdx.x / SPLIT, i0 = first + 2 * t;
     const float4 alo = slo[0][t + R / 2], ahi = shi[0][t + R / 2], blo = slo[1][t + R / 2], bhi = shi[1][t + R / 2];
-    float best0 = INFINITY, best1 = INFINITY;
-    int m0 = 2 * R + 2, m1 = 2 * R + 2;   // candidate's place: twice the step plus the parity (none: beyond the last)
-    // positions i0 - R .. i0 + R + 1: the first is out of the second cluster's reach, the
-    // last out of the first's, and neither is its own neighbour
-    auto step = [&](int m, bool e0, bool e1, bool o0, bool o1) {
+    float best0 = merged_area(alo, ahi, blo, bhi), best1;
+    int m0 = R + 1, m1 = R;   // candidate's place: twice the step plus the parity (none: beyond the last)
+    if (!(best0 < INFINITY)) { best0 = INFINITY; m0 = m1 = 2 * R + 2; }
+    best1 = best0;
+    // positions i0 - R .. i0 + R + 1 but the two clusters' own: the first is out of the second
+    // cluster's reach, the last out of the first's
+    auto step = [&](int m, bool e1, bool o0) {
         const float4 elo = slo[0][t + m], ehi = shi[0][t + m];
-        if (e0) { const float a = merged_area(alo, ahi, elo, ehi); if (a < best0) { best0 = a; m0 = 2 * m; } }
+        { const float a = merged_area(alo, ahi, elo, ehi); if (a < best0) { best0 = a; m0 = 2 * m; } }
         if (e1) { const float a = merged_area(blo, bhi, elo, ehi); if (a < best1) { best1 = a; m1 = 2 * m; } }
         const float4 olo = slo[1][min(t + m, kHalf - 1)], ohi = shi[1][min(t + m, kHalf - 1)];
         if (o0) { const float a = merged_area(alo, ahi, olo, ohi); if (a < best0) { best0 = a; m0 = 2 * m + 1; } }
-        if (o1) { const float a = merged_area(blo, bhi, olo, ohi); if (a < best1) { best1 = a; m1 = 2 * m + 1; } }
+        { const float a = merged_area(blo, bhi, olo, ohi); if (a < best1) { best1 = a; m1 = 2 * m + 1; } }
     };
     if (SPLIT == 1) {
-        step(0, true, false, true, true);
+        step(0, false, true);
 #pragma unroll 4
-        for (int m = 1; m < R / 2; m++) step(m, true, true, true, true);
-        step(R / 2, false, true, true, false);
+        for (int m = 1; m < R / 2; m++) step(m, true, true);
 #pragma unroll 4
-        for (int m = R / 2 + 1; m < R; m++) step(m, true, true, true, true);
-        step(R, true, true, false, true);
+        for (int m = R / 2 + 1; m < R; m++) step(m, true, true);
+        step(R, true, false);
     } else {
-        for (int m = (int)threadIdx.x % SPLIT; m <= R; m += SPLIT) step(m, m != R / 2, m != 0, m != R, m != R / 2);
+        for (int m = (int)threadIdx.x % SPLIT; m <= R; m += SPLIT)
+            if (m != R / 2) step(m, m != 0, m != R);
 #pragma unroll
         for (int d = 1; d < SPLIT; d <<= 1) {
             const float a0 = __shfl_xor_sync(0xFFFFFFFFu, best0, d), a1 = __shfl_xor_sync(0xFFFFFFFFu, best1, d);
@@ -1118,6 +1123,10 @@ __global__ void __launch_bounds__(1024) k_ploc_tail(uint32_t* n_ptr, const float
             uint32_t bj = kInvalid;
             if (c < n) {
                 const float4 alo = lo[c], ahi = hi[c];
+                if ((c ^ 1u) < n) {   // of equal areas the partner, then the lowest position
+                    const float a = merged_area(alo, ahi, lo[c ^ 1u], hi[c ^ 1u]);
+                    if (a < best) { best = a; bj = c ^ 1u; }
+                }
                 const int end = min((int)c + kPlocRadius, (int)n - 1);
                 int j = (int)c - kPlocRadius + (int)sub;
                 if (j < 0) j += (-j + (int)share - 1) / (int)share * (int)share;
