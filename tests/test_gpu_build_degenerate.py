@@ -124,3 +124,18 @@ def _check_world(scenes, inst, rays):
         assert r.stats().error_flags == 0
     for x, y in zip(g, c):
         assert np.array_equal(np.asarray(x).view(np.uint32), np.asarray(y).view(np.uint32))
+
+
+@pytest.mark.parametrize("n", [40, 256, 1500, 2100])
+@pytest.mark.parametrize("kind", ["nested", "far"])
+def test_instances_that_do_not_cluster(kind, n, monkeypatch):
+    """Boxes inside one another, of which a clustering makes a chain, and boxes whose merged
+    areas overflow, which it cannot order."""
+    monkeypatch.setenv("XR_TLAS_BUILDER", "ploc")
+    rng = np.random.default_rng(n)
+    scene = box_scene(rng, 6, 2.0)
+    if kind == "nested":
+        inst = [(0, affine(np.eye(3) * (1.0 + k / 64.0), [0, 0, 0])) for k in rng.permutation(n)]
+    else:
+        inst = [(0, affine(np.eye(3), list(rng.uniform(-1e20, 1e20, 3) * (k > 3)))) for k in range(n)]
+    _check_world([scene], inst, random_rays(rng, 300, -4, 4))

@@ -933,6 +933,10 @@ constexpr int kPlocRadius = XR_PLOC_RADIUS;
 constexpr int kPlocBlock = 256;       // k_ploc_nn: two clusters per thread
 constexpr uint32_t kPlocWide = 1u << 16;   // up to this many: several lanes per cluster
 constexpr uint32_t kPlocTail = 2048;  // clusters that one block takes to the end
+// Where a build may give up for the radix tree (WideBuild::max_depth): a batch of rounds, or one
+// of the last rounds, that merges less than one cluster in this many (boxes in random places
+// lose about one in six a round, boxes inside one another one in 64).
+constexpr uint32_t kPlocFew = 32;
 
 // A cluster: {lo, reference}, {hi, primitives}.
 __global__ void k_ploc_init(uint32_t n, const uint32_t* __restrict__ sorted, const float4* __restrict__ tlo,
@@ -1102,7 +1106,8 @@ __global__ void __launch_bounds__(256) k_ploc_compact(const uint32_t* n_ptr, uin
 // As clusters get fewer, more lanes share the search of one.
 constexpr size_t kPlocTailSmem = kPlocTail * (2 * sizeof(float4) + sizeof(uint32_t));
 __global__ void __launch_bounds__(1024) k_ploc_tail(uint32_t* n_ptr, const float4* __restrict__ clo,
-                                                    const float4* __restrict__ chi, BuildWords* words, PlocTree T) {
+                                                    const float4* __restrict__ chi, BuildWords* words, PlocTree T,
+                                                    bool may_stop) {
     extern __shared__ float4 tail_mem[];
     float4 *lo = tail_mem, *hi = tail_mem + kPlocTail;
     uint32_t* nn = reinterpret_cast<uint32_t*>(tail_mem + 2 * kPlocTail);
@@ -1176,7 +1181,7 @@ __global__ void __launch_bounds__(1024) k_ploc_tail(uint32_t* n_ptr, const float
             out += all;
             __syncthreads();
         }
-        if (out == n) break;   // no progress (infinite areas): `made` will not match
+        if (out == n || (may_stop && n - out < n / kPlocFew)) break;   // little or no progress (infinite areas): `made` will not match
         n = out;
     }
     if (t == 0u) {
@@ -1236,7 +1241,9 @@ inline void sfree(Context* ctx, void* p) { pool_free(ctx, p); }
 
 }  // namespace
 
-xr_status build_wide(Context* ctx, WideBuild& B) {
+// `declined` non-null: a clustering that makes little progress or gives a tree deeper than
+// B.max_depth sets it, and nothing is built.
+static xr_status build_tree(Context* ctx, WideBuild& B, bool* declined) {
     cudaStream_t st = ctx->stream;
     const uint32_t n = B.n;
     const bool records = B.records != nullptr;
@@ -1362,13 +1369,15 @@ xr_status build_wide(Context* ctx, WideBuild& B) {
                 uint32_t left_over = 0;
                 cudaMemcpyAsync(&left_over, &words->clusters[side], 4, cudaMemcpyDeviceToHost, st);
                 if ((s = cuda_check(ctx, cudaStreamSynchronize(st), "bvh: ploc"))) break;
+                if (declined && cnt - left_over < cnt / kPlocFew) { *declined = true; goto done; }
                 if (left_over >= cnt) s = fail(ctx, XR_ERR_STATE, "bvh: clustering made no progress");
                 cnt = left_over;
             }
             if (s) goto done;
             if ((s = cuda_check(ctx, cudaFuncSetAttribute(k_ploc_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                           (int)kPlocTailSmem), "bvh: ploc"))) goto done;
-            k_ploc_tail<<<1, 1024, kPlocTailSmem, st>>>(&words->clusters[side], clo, chi, words, T);
+            k_ploc_tail<<<1, 1024, kPlocTailSmem, st>>>(&words->clusters[side], clo, chi, words, T,
+                                                           declined != nullptr);
         }
         cudaMemsetAsync(sah_flags, 0, (nd + 1) * 4, st);
         if (sah) {
@@ -1400,6 +1409,7 @@ xr_status build_wide(Context* ctx, WideBuild& B) {
             cudaMemcpyAsync(&bflag, flags + nint, 4, cudaMemcpyDeviceToHost, st);
             cudaMemcpyAsync(&dflag, sah_flags + nd, 4, cudaMemcpyDeviceToHost, st);
             if ((s = cuda_check(ctx, cudaStreamSynchronize(st), "bvh: collapse"))) goto done;
+            if (declined && ploc && (back.made != n - 1 || back.level_count[B.max_depth])) { *declined = true; goto done; }
             if (ploc && back.made != n - 1) {
                 s = fail(ctx, XR_ERR_STATE, "bvh: clustering built the wrong number of nodes");
                 goto done;
@@ -1431,11 +1441,21 @@ xr_status build_wide(Context* ctx, WideBuild& B) {
 done:
     sfree(ctx, scratch);
     cudaEventDestroy(e0); cudaEventDestroy(e1);
-    if (s != XR_OK) {
+    if (s != XR_OK || (declined && *declined)) {
         if (!B.slots_into) cudaFree(B.slots);
         if (!B.nodes_into) cudaFree(B.nodes);
         B.slots = nullptr; B.nodes = nullptr;
         B.level_off.clear();
+    }
+    return s;
+}
+
+xr_status build_wide(Context* ctx, WideBuild& B) {
+    bool declined = false;
+    xr_status s = build_tree(ctx, B, B.max_depth ? &declined : nullptr);
+    if (!s && declined) {
+        B.builder = 2;
+        s = build_tree(ctx, B, nullptr);
     }
     return s;
 }

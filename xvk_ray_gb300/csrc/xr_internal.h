@@ -250,6 +250,7 @@ struct WideBuild {
     const uint32_t* ref_prim = nullptr;   // box input of triangle pieces: the triangle of each box
     int emin_floor = -1000;             // lower bound of the finest grid exponent
     int builder = 0;                    // 0: XR_BVH_BUILDER (PLOC unless "lbvh"), 1: PLOC, 2: LBVH
+    uint32_t max_depth = 0;             // non-zero: a PLOC tree of more levels, or slow to make, is built as LBVH instead
     // Caller's arrays to build into (capacity max(n - 1, 1) nodes and 4 n slot words); the build allocates its
     // own when they are null.
     WideNode* nodes_into = nullptr;
