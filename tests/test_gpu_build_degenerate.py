@@ -139,3 +139,20 @@ def test_instances_that_do_not_cluster(kind, n, monkeypatch):
     else:
         inst = [(0, affine(np.eye(3), list(rng.uniform(-1e20, 1e20, 3) * (k > 3)))) for k in range(n)]
     _check_world([scene], inst, random_rays(rng, 300, -4, 4))
+
+
+@pytest.mark.parametrize("n", [1380, 1340])
+def test_deep_chains_are_built(n):
+    """Triangles inside one another cluster one by one: the deepest trees that are built have
+    200 levels (these some 197 and 191), and rays that stay outside find them empty."""
+    s = (1.0 + np.arange(n) / 64.0)[:, None, None]
+    tri = s * np.array([[[-1.0, -1.0, -1.0], [1.0, 1.0, -1.0], [0.0, 0.0, 1.0]]])
+    rays = random_rays(np.random.default_rng(n), 300, 30, 40)
+    rays[:, 4:7] = np.abs(rays[:, 4:7])
+    with xr.Renderer(8, 8) as r:
+        r.upload_scene(_alone(tri))
+        r.build_bvh()
+        p, _, _ = r.trace(rays)
+        st = r.stats()
+    assert 185 <= st.bvh_depth <= 200 and (st.bvh_depth > 192) == (n == 1380)
+    assert st.error_flags == 0 and np.all(p == -1)

@@ -57,7 +57,8 @@ __host__ __device__ __forceinline__ float o2f(uint32_t u) {
 }
 
 // Words of one build on the device: what the kernels share and the host reads back once.
-constexpr uint32_t kBuildLevels = 208;
+constexpr uint32_t kMaxLevels = 200;               // wide levels of a tree
+constexpr uint32_t kBuildLevels = kMaxLevels + 8;
 struct BuildWords {
     uint32_t bounds[8];        // [0..2] centroid min, [3..5] centroid max (ordered), [6] largest |coordinate|
     uint32_t counters[4];      // [0] wide nodes, [1] triangle slots, [3] inconsistencies found
@@ -1416,8 +1417,8 @@ static xr_status build_tree(Context* ctx, WideBuild& B, bool* declined) {
             }
             if (back.counters[3] || bflag || dflag) { s = fail(ctx, XR_ERR_STATE, "bvh: inconsistent radix tree"); goto done; }
             if (back.level_count[level] == 0u) break;
-            if (level + 8u > 200u) { s = fail(ctx, XR_ERR_OVERFLOW, "bvh: collapse did not terminate"); goto done; }
-            until = level + 8u;
+            if (level >= kMaxLevels) { s = fail(ctx, XR_ERR_OVERFLOW, "bvh: collapse did not terminate"); goto done; }
+            until = std::min(level + 8u, kMaxLevels);
         }
         if (back.counters[1] != n) { s = fail(ctx, XR_ERR_STATE, "bvh: triangle slots do not match the primitive count"); goto done; }
         // the nodes each level allocated are the next level
