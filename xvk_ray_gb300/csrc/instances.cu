@@ -287,7 +287,7 @@ xr_status rebuild_tlas(Context* c) {
     wb.builder = n >= 32u && (uint64_t)c->N >= 4096ull * n ? 1 : 2;
     if (const char* e = getenv("XR_TLAS_BUILDER")) wb.builder = strcmp(e, "ploc") == 0 ? 1 : 2;
     // Boxes inside one another cluster into a chain, boxes too large for an area not at all, and
-    // a ray's stack holds 40 groups for both levels: the radix tree splits those by their codes
+    // a ray's stack holds some 40 groups for both levels: the radix tree splits those by their codes
     // (setting 256 boxes inside one another 615 us, of which the clustering that is given up 125).
     // (Levels of a clustered tree: 5 over 2100 boxes in random places, 13 over 1M triangles.)
     wb.max_depth = 16;

@@ -89,7 +89,11 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
 // Per-warp working set of the traversal in shared memory: the queue of triangle tests,
 // and per lane its ray as the triangle test wants it and the closest hit so far.
 constexpr uint32_t kTriQueue = 64;
-constexpr uint32_t kStackRing = 64;   // at most kStackSize groups are on a lane's stack
+constexpr uint32_t kStackRing = 64;
+// Groups a lane's stack may hold.  A ray that enters an instance saves the next top-level node
+// beside the rest of that node's group: one entry more than the group alone.
+template <bool INST> constexpr uint32_t kStackMax = (uint32_t)kStackSize + (INST ? 1u : 0u);
+static_assert(kStackMax<true> <= kStackRing, "the stack is a ring of this many");
 template <bool INST>
 struct alignas(16) TraceWarp {
     float4 ray0[32];             // the origin's components kx, ky, kz; tmin
@@ -200,7 +204,7 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
         e.y &= e.y - 1u;
         cur = e.x + __popc((e.y >> 8) & ((1u << (k ^ flip)) - 1u));
         if (e.y & 0xFFu) {
-            if (sp - sb < (uint32_t)kStackSize) slot_of(sp++, tail) = e;
+            if (sp - sb < kStackMax<INST>) slot_of(sp++, tail) = e;
             else overflow();
         }
     };
@@ -493,7 +497,7 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
                         found.y &= ~(1u << (s1 ^ flip));
                         cur = w1.x + __popc((w1.z >> 24) & ((1u << s1) - 1u));
                         if (found.y & 0xFFu) {
-                            if (sp - sb < (uint32_t)kStackSize) slot_of(sp++, tail) = found;
+                            if (sp - sb < kStackMax<INST>) slot_of(sp++, tail) = found;
                             else overflow();
                         }
                         found.y = 0u;
@@ -523,7 +527,7 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
             m &= 0u - m;
             const uint32_t slot = w1.y + __popc(w1.z & (m - 1u));
             tg_mask ^= m;
-            if (slot >= sc.n_inst_slots || sp + 3u > (uint32_t)kStackSize) {
+            if (slot >= sc.n_inst_slots || sp + 3u > kStackMax<INST>) {
                 overflow();
                 tg_mask = 0u;
             } else {
