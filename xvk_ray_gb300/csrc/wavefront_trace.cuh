@@ -34,25 +34,12 @@ namespace xr {
 
 constexpr uint32_t kTriGroupBit = 0x80000000u;   // stack entry holds a group of instances (two-level traversal)
 constexpr uint32_t kLevelBit = 0x40000000u;      // stack entry marks the return to the top-level BVH
-#ifndef XR_REFILL_MIN
-#define XR_REFILL_MIN 8
-#endif
 #ifndef XR_MIN_RUNNING
 #define XR_MIN_RUNNING 16
 #endif
 #ifndef XR_ENTER_MIN
 #define XR_ENTER_MIN 4
 #endif
-// Default: queued triangle tests that make a batch.  A two-level ray waits for its tests
-// before it leaves an instance, so the batch is smaller (dynamic world, 256 instances, three
-// renderers alternating: 6.42 ms a frame with 32, 6.29 with 24, 6.30 with 16).
-template <bool INST> constexpr uint32_t kTestBatch = INST ? 16u : 32u;
-// Default: finished lanes before a refill.  Rays end soon in a small tree, so a refill (some
-// 200 instructions) serves more lanes there; in a large one idle lanes cost more.  Frames of
-// three contexts at 1600 x 1000, 8 and 20: 2.4k nodes 700 / 666 us, 4.8k 766 / 736, 9.7k
-// 883 / 858, 19k 958 / 954; 853 x 479 over 14k nodes 197 / 203, 1080p over 163k 1616 / 1659.
-constexpr uint32_t kRefillMin = XR_REFILL_MIN;
-constexpr uint32_t kRefillMinSmall = 20, kSmallTree = 12288;   // nodes
 constexpr uint32_t kMinRunning = XR_MIN_RUNNING;   // fewer lanes with nodes to visit: test what is queued
 constexpr uint32_t kEnterMin = XR_ENTER_MIN;       // lanes that want an instance before they enter together
 constexpr float kMinDir = 1e-20f;                 // smallest direction component seen by the box test
@@ -146,8 +133,8 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
     constexpr uint32_t FULL = 0xFFFFFFFFu;
     uint32_t n_visits = 0, n_tests = 0;
     // queue tuning of the context (0: the defaults)
-    const uint32_t refill_min = sc.refill_min ? sc.refill_min : !INST && sc.n_nodes < kSmallTree ? kRefillMinSmall : kRefillMin;
-    const uint32_t batch = sc.postpone_below ? sc.postpone_below : kTestBatch<INST>;
+    const uint32_t refill_min = sc.refill_min ? sc.refill_min : default_refill(INST, sc.n_nodes);
+    const uint32_t batch = sc.postpone_below ? sc.postpone_below : default_batch(INST);
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt_mask = (1u << lane) - 1u;
     uint32_t q_head = 0, q_count = 0;   // the queue, a ring; these are the same in all lanes

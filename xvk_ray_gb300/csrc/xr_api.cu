@@ -852,13 +852,19 @@ xr_status xr_autotune(XrContext* c, const XrUniformBufferObject* ubos, uint32_t 
             if (x >= 1 && x != occ && std::find(v.begin(), v.end(), (uint32_t)x) == v.end()) v.push_back((uint32_t)x);
         return v;
     };
+    // the values of a knob whose default (tried as 0) depends on the scene
+    const bool inst = !c->instances.empty();
+    auto but = [](std::vector<uint32_t> v, uint32_t dflt) {
+        v.erase(std::remove(v.begin(), v.end(), dflt), v.end());
+        return v;
+    };
     // coordinate descent: each knob in turn takes the value with the shortest frames, the
     // others held at the best so far (0 = the built-in default of every knob)
     std::vector<Knob> knobs = {
         {&c->tune_trace_ctas, fractions(occ_t)},                       // persistent traversal CTAs per SM
         {&c->tune_shade_ctas, fractions(occ_s)},                       // persistent shading CTAs per SM
-        {&c->tune_refill, {0u, 4u, 6u, 12u, 16u}},                     // ray-queue refill: idle lanes per fetch
-        {&c->tune_postpone, {0u, 8u, 16u, 24u}},                       // queued triangle tests that make a batch
+        {&c->tune_refill, but({0u, 4u, 6u, 8u, 12u, 16u, 20u}, default_refill(inst, c->n_nodes))},   // ray-queue refill: idle lanes per fetch
+        {&c->tune_postpone, but({0u, 8u, 16u, 24u, 32u}, default_batch(inst))},   // queued triangle tests that make a batch
         {&c->tune_bundle, {0u, 1u, 2u}},                               // camera-ray bundle: 8x4, 16x2, 4x8 pixels
         {&c->tune_temporal_block, {0u, 32u, 128u, 256u}},              // temporal pass block (default 64)
         {&c->tune_spatial_block, {0u, 64u, 256u}},                     // spatial passes' block (default 128)

@@ -92,6 +92,25 @@ __host__ __device__ inline void set_cells(WideNode& n, const int e[3]) {
     n.cell_z = cell_exponent(e[2]) << 23;
 }
 
+// Defaults of the traversal's queues (xr_set_tuning and xr_autotune change them).
+#ifndef XR_REFILL_MIN
+#define XR_REFILL_MIN 8
+#endif
+constexpr uint32_t kRefillMin = XR_REFILL_MIN, kRefillMinSmall = 20, kSmallTree = 12288;   // lanes, lanes, nodes
+// Finished lanes before a refill.  A refill (some 200 instructions) serves more lanes where rays
+// end soon; where they go on for long, idle lanes cost more.  Frames of three contexts at
+// 1600 x 1000, 8 and 20: 2.4k nodes 700 / 666 us, 4.8k 766 / 736, 9.7k 883 / 858, 19k 958 / 954;
+// 853 x 479 over 14k nodes 197 / 203, 1080p over 163k 1616 / 1659.  The node count stands for the
+// length of a ray, and only roughly: between 10k and 20k nodes both values are within 3%, the
+// smaller frame wanting 8.
+__host__ __device__ constexpr uint32_t default_refill(bool instances, uint32_t nodes) {
+    return !instances && nodes < kSmallTree ? kRefillMinSmall : kRefillMin;
+}
+// Queued triangle tests that make a batch.  A two-level ray waits for its tests before it leaves
+// an instance, so the batch is smaller (dynamic world of 256 instances, three contexts: 6.42 ms a
+// frame with 32, 6.29 with 24, 6.30 with 16 when the queue came in; 16 and 24 alike since).
+__host__ __device__ constexpr uint32_t default_batch(bool instances) { return instances ? 16u : 32u; }
+
 struct DeviceScene {
     const float4* tri;        // 3 float4 per BVH triangle slot: v0 {xyz, prim id}, v1, v2
     const WideNode* nodes;
