@@ -64,6 +64,7 @@ struct BuildWords {
     uint32_t counters[4];      // [0] wide nodes, [1] triangle slots, [3] inconsistencies found
     uint32_t clusters[2];      // clusters left, by parity of the clustering round
     uint32_t made;             // binary nodes made by the clustering
+    uint32_t stalled;          // a round of it has merged few clusters
     uint32_t root;             // root of the binary tree
     uint32_t level_count[kBuildLevels];   // wide nodes of each level
 };
@@ -922,11 +923,13 @@ __global__ void k_esc(const uint4* __restrict__ tri_idx, const float4* __restric
 // Morton order; each finds the cluster within +-kPlocRadius positions whose
 // merged box has the smallest surface area, mutual pairs merge into a new
 // internal node at the lower position, the array is compacted, and rounds repeat
-// until one cluster is left.  Of equal areas the partner (positions 2k and 2k + 1)
-// comes first, then the pairs by their indices: the globally best pair is always
-// mutual, so every round merges, and boxes that coincide or stand in a regular row
-// halve in a round (by the indices alone 256 equal boxes merged one pair a round into
-// a chain of 255 nodes, a row of 256 took 135 rounds; 8 and 8).
+// until one cluster is left.  Of equal areas the pairs go by their indices: the globally
+// best pair is always mutual, so every round merges.  Boxes that coincide or stand in a
+// regular row have so many equal areas that a round merges next to nothing (256 equal
+// boxes: one pair a round, a chain of 255 nodes; a row of 256: 135 rounds).  From the first
+// round on that merges few clusters (ploc_few) the partner (positions 2k and 2k + 1) comes
+// first among equals, which keeps the best pair mutual and halves such boxes in a round;
+// trees whose rounds never stall are those of the indices alone.
 #ifndef XR_PLOC_RADIUS
 #define XR_PLOC_RADIUS 64
 #endif
@@ -934,10 +937,11 @@ constexpr int kPlocRadius = XR_PLOC_RADIUS;
 constexpr int kPlocBlock = 256;       // k_ploc_nn: two clusters per thread
 constexpr uint32_t kPlocWide = 1u << 16;   // up to this many: several lanes per cluster
 constexpr uint32_t kPlocTail = 2048;  // clusters that one block takes to the end
-// Where a build may give up for the radix tree (WideBuild::max_depth): a batch of rounds, or one
-// of the last rounds, that merges less than one cluster in this many (boxes in random places
-// lose about one in six a round, boxes inside one another one in 64).
-constexpr uint32_t kPlocFew = 32;
+// Few of n clusters merged in a round: boxes in random places lose about one in six, equal
+// boxes one pair, a row of boxes or boxes inside one another one in 64.
+__host__ __device__ __forceinline__ bool ploc_few(uint32_t n, uint32_t merged) {
+    return n > 16u && merged < (n < 64u ? 2u : n / 32u);
+}
 
 // A cluster: {lo, reference}, {hi, primitives}.
 __global__ void k_ploc_init(uint32_t n, const uint32_t* __restrict__ sorted, const float4* __restrict__ tlo,
@@ -959,16 +963,18 @@ __device__ __forceinline__ float merged_area(float4 alo, float4 ahi, float4 blo,
 // What stands for a position outside the array: its merged area is infinite, so it never wins.
 __device__ __forceinline__ float4 nowhere(float s) { return make_float4(s * INFINITY, s * INFINITY, s * INFINITY, 0.0f); }
 
-// Nearest neighbours.  The partner is taken first, then the candidates in ascending order
-// with a strict comparison: of equal areas the partner wins, then the lowest position, which
-// orders the other pairs by area, lower index, upper index.  A thread searches for two adjacent clusters, so that each candidate read from
-// shared memory serves two (reading it was the bound: 128 x 32 B per cluster); even and
-// odd positions are stored apart, so that the threads' reads are consecutive.  SPLIT > 1:
+// Nearest neighbours.  Candidates are taken in ascending order with a strict comparison:
+// of equal areas the lowest position wins, which orders pairs by area, lower index, upper
+// index; once rounds have stalled the partner is taken before.  A thread searches for two
+// adjacent clusters, so that each candidate read from shared memory serves two (reading it
+// was the bound: 128 x 32 B per cluster); even and odd positions are stored apart, so that
+// the threads' reads are consecutive.  SPLIT > 1:
 // that many lanes share a pair's candidates, for counts that leave the chip idle and the
 // search a serial chain (2048 .. 64K clusters: 10.5 us a round with one lane, 5.5 with 8).
 template <int SPLIT>
-__global__ void __launch_bounds__(kPlocBlock) k_ploc_nn(const uint32_t* n_ptr, const float4* __restrict__ clo,
-                                                        const float4* __restrict__ chi, uint32_t* __restrict__ nn) {
+__global__ void __launch_bounds__(kPlocBlock) k_ploc_nn(const uint32_t* n_ptr, const uint32_t* stalled,
+                                                        const float4* __restrict__ clo, const float4* __restrict__ chi,
+                                                        uint32_t* __restrict__ nn) {
     constexpr int R = kPlocRadius, kPairs = kPlocBlock / SPLIT, kHalf = kPairs + R;
     static_assert(R % 2 == 0, "even and odd candidates are stored apart");
     __shared__ float4 slo[2][kHalf], shi[2][kHalf];
@@ -984,30 +990,32 @@ __global__ void __launch_bounds__(kPlocBlock) k_ploc_nn(const uint32_t* n_ptr, c
     __syncthreads();
     const int t = threadIdx.x / SPLIT, i0 = first + 2 * t;
     const float4 alo = slo[0][t + R / 2], ahi = shi[0][t + R / 2], blo = slo[1][t + R / 2], bhi = shi[1][t + R / 2];
-    float best0 = merged_area(alo, ahi, blo, bhi), best1;
-    int m0 = R + 1, m1 = R;   // candidate's place: twice the step plus the parity (none: beyond the last)
-    if (!(best0 < INFINITY)) { best0 = INFINITY; m0 = m1 = 2 * R + 2; }
-    best1 = best0;
-    // positions i0 - R .. i0 + R + 1 but the two clusters' own: the first is out of the second
-    // cluster's reach, the last out of the first's
-    auto step = [&](int m, bool e1, bool o0) {
+    float best0 = INFINITY, best1 = INFINITY;
+    int m0 = 2 * R + 2, m1 = 2 * R + 2;   // candidate's place: twice the step plus the parity (none: beyond the last)
+    if (*stalled) {
+        const float a = merged_area(alo, ahi, blo, bhi);
+        if (a < INFINITY) { best0 = best1 = a; m0 = R + 1; m1 = R; }
+    }
+    // positions i0 - R .. i0 + R + 1: the first is out of the second cluster's reach, the
+    // last out of the first's, and neither is its own neighbour
+    auto step = [&](int m, bool e0, bool e1, bool o0, bool o1) {
         const float4 elo = slo[0][t + m], ehi = shi[0][t + m];
-        { const float a = merged_area(alo, ahi, elo, ehi); if (a < best0) { best0 = a; m0 = 2 * m; } }
+        if (e0) { const float a = merged_area(alo, ahi, elo, ehi); if (a < best0) { best0 = a; m0 = 2 * m; } }
         if (e1) { const float a = merged_area(blo, bhi, elo, ehi); if (a < best1) { best1 = a; m1 = 2 * m; } }
         const float4 olo = slo[1][min(t + m, kHalf - 1)], ohi = shi[1][min(t + m, kHalf - 1)];
         if (o0) { const float a = merged_area(alo, ahi, olo, ohi); if (a < best0) { best0 = a; m0 = 2 * m + 1; } }
-        { const float a = merged_area(blo, bhi, olo, ohi); if (a < best1) { best1 = a; m1 = 2 * m + 1; } }
+        if (o1) { const float a = merged_area(blo, bhi, olo, ohi); if (a < best1) { best1 = a; m1 = 2 * m + 1; } }
     };
     if (SPLIT == 1) {
-        step(0, false, true);
+        step(0, true, false, true, true);
 #pragma unroll 4
-        for (int m = 1; m < R / 2; m++) step(m, true, true);
+        for (int m = 1; m < R / 2; m++) step(m, true, true, true, true);
+        step(R / 2, false, true, true, false);
 #pragma unroll 4
-        for (int m = R / 2 + 1; m < R; m++) step(m, true, true);
-        step(R, true, false);
+        for (int m = R / 2 + 1; m < R; m++) step(m, true, true, true, true);
+        step(R, true, true, false, true);
     } else {
-        for (int m = (int)threadIdx.x % SPLIT; m <= R; m += SPLIT)
-            if (m != R / 2) step(m, m != 0, m != R);
+        for (int m = (int)threadIdx.x % SPLIT; m <= R; m += SPLIT) step(m, m != R / 2, m != 0, m != R, m != R / 2);
 #pragma unroll
         for (int d = 1; d < SPLIT; d <<= 1) {
             const float a0 = __shfl_xor_sync(0xFFFFFFFFu, best0, d), a1 = __shfl_xor_sync(0xFFFFFFFFu, best1, d);
@@ -1080,7 +1088,7 @@ __global__ void __launch_bounds__(1024) k_ploc_merge(const uint32_t* n_ptr, cons
 }
 
 // Closes the gaps between the blocks' clusters; each block adds up the counts before its own.
-__global__ void __launch_bounds__(256) k_ploc_compact(const uint32_t* n_ptr, uint32_t* n_next,
+__global__ void __launch_bounds__(256) k_ploc_compact(const uint32_t* n_ptr, uint32_t* n_next, uint32_t* stalled,
                                                       const uint32_t* __restrict__ sums, const float4* __restrict__ olo,
                                                       const float4* __restrict__ ohi, float4* __restrict__ clo,
                                                       float4* __restrict__ chi) {
@@ -1099,7 +1107,10 @@ __global__ void __launch_bounds__(256) k_ploc_compact(const uint32_t* n_ptr, uin
         clo[before + i] = olo[b * 1024u + i];
         chi[before + i] = ohi[b * 1024u + i];
     }
-    if (b == nb - 1u && threadIdx.x == 0u) *n_next = before + cnt;
+    if (b == nb - 1u && threadIdx.x == 0u) {
+        *n_next = before + cnt;
+        if (ploc_few(*n_ptr, *n_ptr - (before + cnt))) *stalled = 1u;
+    }
 }
 
 // The last rounds, from at most kPlocTail clusters to one, in one block: at 1M primitives
@@ -1118,6 +1129,7 @@ __global__ void __launch_bounds__(1024) k_ploc_tail(uint32_t* n_ptr, const float
     if (n > kPlocTail) return;   // not the host's promise: `made` will not match
     for (uint32_t i = t; i < n; i += 1024u) { lo[i] = clo[i]; hi[i] = chi[i]; }
     if (t == 0u) made = words->made;
+    bool stalled = words->stalled != 0u;   // the same in all threads
     __syncthreads();
     while (n > 1u) {
         uint32_t share = 1u;   // lanes per cluster
@@ -1129,7 +1141,7 @@ __global__ void __launch_bounds__(1024) k_ploc_tail(uint32_t* n_ptr, const float
             uint32_t bj = kInvalid;
             if (c < n) {
                 const float4 alo = lo[c], ahi = hi[c];
-                if ((c ^ 1u) < n) {   // of equal areas the partner, then the lowest position
+                if (stalled && (c ^ 1u) < n) {
                     const float a = merged_area(alo, ahi, lo[c ^ 1u], hi[c ^ 1u]);
                     if (a < best) { best = a; bj = c ^ 1u; }
                 }
@@ -1182,7 +1194,11 @@ __global__ void __launch_bounds__(1024) k_ploc_tail(uint32_t* n_ptr, const float
             out += all;
             __syncthreads();
         }
-        if (out == n || (may_stop && n - out < n / kPlocFew)) break;   // little or no progress (infinite areas): `made` will not match
+        if (out == n) break;   // no progress (infinite areas): `made` will not match
+        if (ploc_few(n, n - out)) {
+            if (stalled && may_stop) break;   // the same
+            stalled = true;
+        }
         n = out;
     }
     if (t == 0u) {
@@ -1361,16 +1377,16 @@ static xr_status build_tree(Context* ctx, WideBuild& B, bool* declined) {
                 for (uint32_t r = 0; r < rounds; r++, side ^= 1u) {
                     uint32_t *cur = &words->clusters[side], *next = &words->clusters[side ^ 1u];
                     if (cnt > kPlocWide)
-                        k_ploc_nn<1><<<(cnt + 2 * kPlocBlock - 1) / (2 * kPlocBlock), kPlocBlock, 0, st>>>(cur, clo, chi, nn);
+                        k_ploc_nn<1><<<(cnt + 2 * kPlocBlock - 1) / (2 * kPlocBlock), kPlocBlock, 0, st>>>(cur, &words->stalled, clo, chi, nn);
                     else
-                        k_ploc_nn<8><<<(cnt + kPlocBlock / 4 - 1) / (kPlocBlock / 4), kPlocBlock, 0, st>>>(cur, clo, chi, nn);
+                        k_ploc_nn<8><<<(cnt + kPlocBlock / 4 - 1) / (kPlocBlock / 4), kPlocBlock, 0, st>>>(cur, &words->stalled, clo, chi, nn);
                     k_ploc_merge<<<(cnt + 1023) / 1024, 1024, 0, st>>>(cur, nn, clo, chi, olo, ohi, sums, &words->made, T);
-                    k_ploc_compact<<<(cnt + 1023) / 1024, 256, 0, st>>>(cur, next, sums, olo, ohi, clo, chi);
+                    k_ploc_compact<<<(cnt + 1023) / 1024, 256, 0, st>>>(cur, next, &words->stalled, sums, olo, ohi, clo, chi);
                 }
                 uint32_t left_over = 0;
                 cudaMemcpyAsync(&left_over, &words->clusters[side], 4, cudaMemcpyDeviceToHost, st);
                 if ((s = cuda_check(ctx, cudaStreamSynchronize(st), "bvh: ploc"))) break;
-                if (declined && cnt - left_over < cnt / kPlocFew) { *declined = true; goto done; }
+                if (declined && ploc_few(cnt, cnt - left_over)) { *declined = true; goto done; }
                 if (left_over >= cnt) s = fail(ctx, XR_ERR_STATE, "bvh: clustering made no progress");
                 cnt = left_over;
             }
