@@ -126,10 +126,6 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
                                                  float retry_tmax = 0.0f) {
     static_assert(!RETRY || !ANY, "the retry is for closest-hit traversal");
     constexpr bool HELP = !INST;
-    // Nearest box first (see the visit): pays where a wrong turn costs an instance entry
-    // (dynamic world 6.82 -> 6.40 ms); in one level the extra instructions cost what the 9%
-    // fewer visits save.
-    constexpr bool NEAR = INST && !ANY;
     constexpr uint32_t FULL = 0xFFFFFFFFu;
     uint32_t n_visits = 0, n_tests = 0;
     // queue tuning of the context (0: the defaults)
@@ -167,7 +163,7 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
     // boxes, so no box holding a hit is culled; the triangle test uses the true direction.
     // The sign bits select the near planes (so that -0 picks the same planes as its
     // infinite reciprocal).  The divisions are correctly rounded: rcp.approx, within an ulp,
-    // would save 2% of the dynamic world's frame and 0.6% of one level's, but the planes'
+    // would save 1.1% of the dynamic world's frame and 0.6% of one level's, but the planes'
     // constants then start from a less exact operand.
     auto set_dir = [&](float3 d) {
         idx = 1.0f / copysignf(fmaxf(fabsf(d.x), kMinDir), d.x);
@@ -194,12 +190,6 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
             if (sp - sb < kStackMax<INST>) slot_of(sp++, tail) = e;
             else overflow();
         }
-    };
-    // A group whose nearest child starts beyond the closest hit has nothing left to find:
-    // the bound is below every child's entry, and the margin is the box test's own.  A bound
-    // of 0 stands for any entry below, so a hit behind the origin drops no group for it.
-    auto beyond = [&](uint2 e) {
-        return __uint_as_float(e.y & 0xFFFF0000u) > fmaxf((h_t * (1.0f + 1e-6f) + 1e-30f) * (1.0f + 2e-6f), 0.0f);
     };
     // The whole ray's start: at the top-level root, or at the root of its scene.
     auto start_ray = [&](uint32_t root) {
@@ -230,8 +220,6 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
                 --sp;
                 e.y = 0u;
                 break;
-            } else if (NEAR && beyond(e)) {
-                e.y = 0u;
             }
             --sp;
         }
@@ -447,7 +435,6 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
                 const uint32_t zn0 = nz ? w4.z : w3.x, zn1 = nz ? w4.w : w3.y;
                 const uint32_t zf0 = nz ? w3.x : w4.z, zf1 = nz ? w3.y : w4.w;
                 uint32_t hm = 0;   // the hit slots' bits of the child mask
-                int32_t near1 = 0x7FFFFFFF, near2 = 0x7FFFFFFF;   // the two nearest hit boxes: entry t, slot in the low bits
 #pragma unroll
                 for (uint32_t i = 0; i < 8; i++) {
                     const float txn = __fmaf_rn(qplane(i < 4 ? xn0 : xn1, i & 3u), sx, ax);
@@ -458,12 +445,7 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
                     const float tzf = __fmaf_rn(qplane(i < 4 ? zf0 : zf1, i & 3u), sz, az);
                     const float tn = fmaxf(max3f(txn, tyn, tzn), tmin_box);
                     const float tf = fminf(min3f(txf, tyf, tzf), tlimit);
-                    const bool box_hit = tn <= __fmaf_rn(tf, 1.0f + 2e-6f, 1e-30f);
-                    if (box_hit) hm |= (7u << (3u * i)) | (1u << (24u + i));
-                    if (!NEAR) continue;
-                    const int32_t key = box_hit ? (__float_as_int(tn) & ~7) | (int32_t)i : 0x7FFFFFFF;
-                    near2 = min(near2, max(near1, key));
-                    near1 = min(near1, key);
+                    if (tn <= __fmaf_rn(tf, 1.0f + 2e-6f, 1e-30f)) hm |= (7u << (3u * i)) | (1u << (24u + i));
                 }
                 // internal hits from slot order to near-to-far order (bit k = slot k ^ flip)
                 hm &= w1.z;
@@ -472,26 +454,8 @@ __device__ __forceinline__ void trace_persistent(TraceWarp<INST>& sh, const Devi
                 if (flip & 2u) ih = ((ih & 0x33u) << 2) | ((ih >> 2) & 0x33u);
                 if (flip & 4u) ih = ((ih & 0x0Fu) << 4) | ((ih >> 4) & 0x0Fu);
                 found = make_uint2(w1.x, ih | ((w1.z >> 16) & 0xFF00u));
-                if (NEAR && ih) {
-                    // The nearest hit box, when it is an internal child, is visited next and the
-                    // second nearest bounds the rest from below; else the first child in octant
-                    // order, and the nearest box is the bound.  (Entries behind the origin are
-                    // ordered backwards as integers: any of them may come first, and the bound is 0.)
-                    const uint32_t s1 = (uint32_t)near1 & 7u;
-                    const bool is_node = (w1.z >> (24u + s1)) & 1u;
-                    found.y |= (uint32_t)max(is_node ? near2 : near1, 0) & 0xFFFF0000u;
-                    if (is_node) {
-                        found.y &= ~(1u << (s1 ^ flip));
-                        cur = w1.x + __popc((w1.z >> 24) & ((1u << s1) - 1u));
-                        if (found.y & 0xFFu) {
-                            if (sp - sb < kStackMax<INST>) slot_of(sp++, tail) = found;
-                            else overflow();
-                        }
-                        found.y = 0u;
-                    }
-                }
                 // children come after their parent, so every descent ends
-                if (ih && w1.x <= node) { overflow(); cur = kInvalid; found.y = 0u; }
+                if (ih && w1.x <= node) { overflow(); found.y = 0u; }
                 tg_base = INST && !in_blas ? node : w1.y;
                 tg_valid = w1.z;
                 tg_mask = hm & 0x00FFFFFFu;
