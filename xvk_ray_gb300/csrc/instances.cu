@@ -106,24 +106,29 @@ void world_box(const ScenePart& p, const float w2o[12], float lo[3], float hi[3]
 }
 
 // Reads part p's root node back and decodes its child boxes: plane = origin + q 2^e
-// per axis (the quantised grid of the node).
+// per axis (the quantised grid of the node).  An infinite cell does not say which of the
+// grids from 2^113 on it stands for: on its axis every child takes the part's vertex bounds,
+// widened by a cell of theirs (a 128th of the extent) as a stored box is by its slack.
 xr_status read_root_boxes(Context* c, ScenePart& p) {
     if (!p.root_boxes.empty() || p.n_nodes == 0) return XR_OK;
     WideNode nd;
     cudaMemcpyAsync(&nd, c->d_nodes + p.node_off, sizeof(nd), cudaMemcpyDeviceToHost, c->stream);
     if (xr_status s = cuda_check(c, cudaStreamSynchronize(c->stream), "root boxes")) return s;
     const double org[3] = {nd.px, nd.py, nd.pz};
-    double cell[3];
     const uint32_t ce[3] = {nd.cell_xy >> 23, (nd.cell_xy >> 7) & 0xFFu, nd.cell_z >> 23};
-    // an infinite cell stands for a grid of 2^113 and more: that of the largest finite box covers it
-    for (int k = 0; k < 3; k++) cell[k] = std::ldexp(1.0, ce[k] < 255u ? (int)ce[k] - 142 : 121);
+    double cell[3], wide[3];
+    for (int k = 0; k < 3; k++) {
+        cell[k] = std::ldexp(1.0, (int)ce[k] - 142);
+        wide[k] = ((double)p.hi[k] - (double)p.lo[k]) / 128.0;
+    }
     for (uint32_t slot = 0; slot < 8; slot++) {
         const uint32_t word = slot < 4 ? 0u : 1u, shift = 8u * (slot & 3u);
         if (!((nd.children >> (24u + slot)) & 1u) && !((nd.children >> (3u * slot)) & 7u)) continue;
-        for (int k = 0; k < 3; k++)
-            p.root_boxes.push_back(org[k] + (ce[k] < 255u ? (double)((nd.q[2 * k + word] >> shift) & 0xFFu) * cell[k] : 0.0));
-        for (int k = 0; k < 3; k++)
-            p.root_boxes.push_back(org[k] + (double)((nd.q[6 + 2 * k + word] >> shift) & 0xFFu) * cell[k]);
+        for (int side = 0; side < 2; side++)
+            for (int k = 0; k < 3; k++) {
+                const double plane = org[k] + (double)((nd.q[6 * side + 2 * k + word] >> shift) & 0xFFu) * cell[k];
+                p.root_boxes.push_back(ce[k] < 255u ? plane : side ? p.hi[k] + wide[k] : p.lo[k] - wide[k]);
+            }
     }
     return XR_OK;
 }
