@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kPrepBlock) k_tri_prep(const uint4* __restrict
         const int k = threadIdx.x;
         float m = part[0][k];
         for (int w = 1; w < kPrepBlock / 32; w++) m = fminf(m, part[w][k]);
-        if (k == 6) atomicMax(&bounds[6], __float_as_uint(-m));
+        if (k == 6) atomicMax(&bounds[6], __float_as_uint(fabsf(m)));   // -m of +0 would be the largest word
         else if (m < INFINITY) {
             if (k < 3) atomicMin(&bounds[k], f2o(m));
             else atomicMax(&bounds[k], f2o(-m));
