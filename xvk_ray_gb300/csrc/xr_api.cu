@@ -369,6 +369,10 @@ xr_status xr_create(const XrDeviceDesc* desc, XrContext** out) {
         uint64_t keep = UINT64_MAX;
         if ((s = cuda_check(c, cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep), "memory pool")))
             goto bad;
+        // the staging memory of host calls, so that the first of them does not grow the pool (95 us)
+        void* stage = nullptr;
+        if ((s = pool_alloc_bytes(c, &stage, kStagePooled, "memory pool"))) goto bad;
+        pool_free(c, stage);
     }
     if ((s = cuda_check(c, cudaMalloc((void**)&c->d_counters, kCounterWords * 4), "counters"))) goto bad;
     if ((s = cuda_check(c, cudaMemset(c->d_counters, 0, kCounterWords * 4), "counters"))) goto bad;
