@@ -141,6 +141,9 @@ enum { XR_DEVFLAG_STACK_OVERFLOW = 1u, XR_DEVFLAG_QUEUE_OVERFLOW = 2u, XR_DEVFLA
 
 /* ---- lifetime: replaces Application/ApplicationRT/ApplicationReSTIRGI construction
         (src/Vulkan/RayTracing/ApplicationReSTIRGI.cpp:25-29) ---- */
+/* A context maps 32 MB of device memory when it is made and keeps it until it is destroyed:
+   the host arrays of ray queries and cache calls are staged there (larger calls allocate
+   their own block and free it). */
 xr_status xr_create(const XrDeviceDesc* desc, XrContext** out);
 void xr_destroy(XrContext* ctx);
 
@@ -227,7 +230,8 @@ xr_status xr_run_pass(XrContext* ctx, const XrUniformBufferObject* ubo, uint32_t
 /* ---- closest-hit / any-hit queries on the built BVH (TraceRay semantics of
         ReSTIRGIInitialSample.rgen.hlsl:90-98 and ReSTIRGISpatialReuse.rgen.hlsl:44-62).
         rays: n x 8 floats {o.xyz, tmin, d.xyz, tmax} in host memory.  prim = -1 on
-        miss; t and bary (b1, b2) are written on a hit.  Ties: lowest primitive id. */
+        miss; t and bary (b1, b2) are written on a hit.  Ties: lowest primitive id.
+        tmin may be negative: the closest hit is the one of the smallest t. */
 xr_status xr_trace_rays(XrContext* ctx, const float* rays, uint32_t n, int32_t any_hit,
                         int32_t* prim, float* t, float* bary);
 /* Same on device pointers, asynchronous on the context stream. */
@@ -342,7 +346,8 @@ typedef struct XrTuning {
     float ms_default;            /* xr_autotune: the all-defaults configuration */
     uint32_t configs_tried;
     /* ray queues of the persistent traversal: a warp refills from its queue once this many
-       lanes are idle (default 8, in trees of fewer than 12288 nodes 20), and tests triangles once this many are queued (default 32, with instances 16) */
+       lanes are idle (default 8, in trees of fewer than 12288 nodes 20), and tests triangles
+       once this many are queued (default 32, with instances 16) */
     uint32_t refill_min, postpone_below;
     uint32_t ray_bundle;         /* camera rays of a 16 x 8 tile per warp: 0 8x4 blocks (default), 1 16x2 rows, 2 4x8 */
     uint32_t temporal_block;     /* threads per block of the temporal pass: 32, 64 (default), 128, 256 */

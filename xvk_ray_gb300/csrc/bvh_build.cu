@@ -14,9 +14,10 @@
 //      bounds bottom-up, the second arrival at a node computing its box
 //   5. the SAH decisions of the collapse, bottom-up
 //   6. top-down collapse, one level per launch, eight lanes per wide node: the children the
-//      decisions give, children of <= 3 triangles become leaves, slots are assigned by
-//      octant of the child centre so that a ray visits near children first, boxes are
-//      quantised to 8 bits (rounded outwards, plus the slack of kBoxSlackCells).
+//      decisions give, children of <= 3 triangles become leaves, children and slots are paired
+//      by how far the child's centre lies towards the slot's octant so that a ray visits near
+//      children first, boxes are quantised to 8 bits (rounded outwards, plus the slack of
+//      kBoxSlackCells).
 // The kernels hand their counts on through device words (BuildWords); the host waits once
 // per batch of clustering rounds and once per batch of levels.
 #include <algorithm>

@@ -286,9 +286,10 @@ xr_status rebuild_tlas(Context* c) {
     wb.records = d_rec;
     // PLOC's tree takes less traversal, the Karras radix tree less time to build (0.11 / 0.11 ms
     // for 3 instances, 0.18 / 0.15 for 65, 0.24 / 0.19 for 201, 0.91 / 0.43 for 8193), so PLOC
-    // where a frame has rays enough for it.  Frames in a world moving every frame, PLOC / Karras:
-    // 256 instances at 1920 x 1080 5.69 / 5.91 ms, 64 at 1280 x 720 2.14 / 2.20, 16 there 0.934
-    // / 0.932, 1024 there 4.18 / 4.17, 8192 there 10.98 / 10.81, 200 at 320 x 256 0.61 / 0.59.
+    // where a frame has rays enough for it.  Frames in a world moving every frame, three contexts,
+    // PLOC / Karras: 256 instances at 1920 x 1080 5.52 / 5.58 ms (one context 6.50 / 7.03), 32
+    // there 2.49 / 2.56, 64 at 1280 x 720 1.64 / 1.73, 16 there 0.80 / 0.81, 1024 there 3.63 / 3.59,
+    // 8192 there 10.1 / 9.5, 200 at 320 x 256 0.63 / 0.59.
     wb.builder = n >= 32u && (uint64_t)c->N >= 4096ull * n ? 1 : 2;
     if (const char* e = getenv("XR_TLAS_BUILDER")) wb.builder = strcmp(e, "ploc") == 0 ? 1 : 2;
     // Boxes inside one another cluster into a chain, boxes too large for an area not at all, and

@@ -1,7 +1,7 @@
 // trace_noalloc.cu -- batch ray queries that allocate no memory.
 //
-// xr_trace_rays stages the caller's host rays and results through device
-// buffers it allocates on every call.  Some callers cannot allocate device
+// xr_trace_rays stages the caller's host rays and results through a device
+// block it allocates on every call, from the context's memory pool up to 32 MB.  Some callers cannot allocate device
 // memory at the point where they query rays: an engine whose device memory is
 // owned by its own allocator, or a real-time loop in which allocation (an
 // implicit device synchronisation) is forbidden.  xr_trace_rays_noalloc gives

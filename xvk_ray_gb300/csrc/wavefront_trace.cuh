@@ -17,11 +17,12 @@
 // warp's worth is queued (or too few lanes have nodes left to visit), every lane
 // takes one queued test, whichever lane's ray it belongs to.
 //
-// What bounds it is the issue of instructions: 80-85% of the slots, some 460 a round in one
-// level and 920 in two, 24-26 of 32 lanes active (18-23), the BVH served from L1 and L2.
-// With each lane testing its own triangles, postponed below 8 lanes, tests ran at 12-16 lanes:
-// 2M random rays over 1M triangles 531 -> 469 us, 1080p frames of three contexts 2067 ->
-// 1646, the dynamic world 6.69 -> 5.41 ms (all steps since).
+// What bounds it is the issue of instructions: 80-84% of the slots in the long launches, some
+// 540 a round in one level and 750 in two (a frame's instructions over its rounds, with their
+// share of batches, refills and entries), 23-26 of 32 lanes active (18-23), the BVH served from
+// L1 and L2.  With each lane testing its own triangles, postponed below 8 lanes, tests ran at
+// 12-16 lanes: 2M random rays over 1M triangles 532 -> 472 us, 1080p frames of three contexts
+// 2068 -> 1657, the dynamic world 6.72 -> 5.10 ms (all steps since).
 //
 // The triangle test and the box test are those of traverse.cuh (same arithmetic
 // as the CPU oracle); only the order of the work differs, which the closest-hit

@@ -99,16 +99,17 @@ __host__ __device__ inline void set_cells(WideNode& n, const int e[3]) {
 constexpr uint32_t kRefillMin = XR_REFILL_MIN, kRefillMinSmall = 20, kSmallTree = 12288;   // lanes, lanes, nodes
 // Finished lanes before a refill.  A refill (some 200 instructions) serves more lanes where rays
 // end soon; where they go on for long, idle lanes cost more.  Frames of three contexts at
-// 1600 x 1000, 8 and 20: 2.4k nodes 700 / 666 us, 4.8k 766 / 736, 9.7k 883 / 858, 19k 958 / 954;
-// 853 x 479 over 14k nodes 197 / 203, 1080p over 163k 1616 / 1659.  The node count stands for the
-// length of a ray, and only roughly: between 10k and 20k nodes both values are within 3%, the
-// smaller frame wanting 8.
+// 1600 x 1000, 8 / 20 lanes: 2.4k nodes 708 / 673 us, 4.7k 781 / 744, 10k 893 / 853, 20k 989 / 968,
+// 41k 1226 / 1216; 853 x 479 over 16k nodes 198 / 204, 1920 x 1080 over 163k 1637 / 1654, 2M random
+// rays there 475 / 528.  The node count stands for how long rays go on, and only roughly: at 16k
+// and 20k nodes the two frames differ by their rays a lane.  The line lies where 20 still gains in
+// every frame measured.
 __host__ __device__ constexpr uint32_t default_refill(bool instances, uint32_t nodes) {
     return !instances && nodes < kSmallTree ? kRefillMinSmall : kRefillMin;
 }
 // Queued triangle tests that make a batch.  A two-level ray waits for its tests before it leaves
-// an instance, so the batch is smaller (dynamic world of 256 instances, three contexts: 6.42 ms a
-// frame with 32, 6.29 with 24, 6.30 with 16 when the queue came in; 16 and 24 alike since).
+// an instance, so the batch is smaller (dynamic world of 256 instances, 8 / 16 / 24 / 32 tests:
+// three contexts 5.54 / 5.59 / 5.64 / 5.71 ms a frame, one 6.66 / 6.52 / 6.50 / 6.63).
 __host__ __device__ constexpr uint32_t default_batch(bool instances) { return instances ? 16u : 32u; }
 
 struct DeviceScene {
